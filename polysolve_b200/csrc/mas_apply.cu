@@ -18,10 +18,12 @@
 //    (update_p): PCG uses z only there and in r . z = r . z0 + (P^T r) . zc.
 //
 // Inverses are stored tile-packed (mas_internal.h): the same N (N + 1) / 2 values as packed upper
-// storage, laid out so a warp reads every 32 x 32 tile conflict-free and uses each value for both
-// y_I += T x_J and y_J += T^T x_I; the transposed sums are combined across lanes with a
-// 31-shuffle reduce-transpose per column tile. Storage is FP64, FP32 or binary16 with one
-// power-of-two scale per matrix (FP32 arithmetic for both reduced formats).
+// storage, in 32 x 32 tiles that shared memory serves without bank conflicts by rows and by columns,
+// so a lane forms its whole row of the product from either side of the diagonal and no sum crosses
+// lanes. Storage is FP64, FP32 or binary16 with one power-of-two scale per matrix (FP32 arithmetic
+// for both reduced formats; binary16 runs on the tensor cores).
+
+#include <type_traits>
 
 #include "mas_common.cuh"
 
@@ -29,9 +31,87 @@ namespace pmas
 {
     namespace
     {
+        // Row 32 t + lane of y = M x for one tile-packed symmetric matrix in shared memory, by one warp.
+        // Left of the diagonal the lane takes its column of the mirrored tiles, one product (and, over
+        // the tiles, one running sum) per row r of a tile, added up as a tree over r; right of it its
+        // own row, four partial sums by column modulo 4 per tile (16-byte reads). The order of the
+        // additions is fixed by the matrix alone.
+        template <int T, class Real>
+        __device__ __forceinline__ Real symv_row(const Real *__restrict__ M, const Real *__restrict__ xs, int t, int lane)
+        {
+            constexpr int VEC = 16 / (int)sizeof(Real), UNITS = 32 / VEC;
+            // Opaque to the compiler: the swizzled offsets are formed here (two integer operations each)
+            // instead of being kept, and spilled, across the caller's loop.
+            asm volatile("" : "+r"(lane));
+            M += t * (t - 1) / 2 * 1024 + t * 528; // column tile t
+            Real c[32];
+#pragma unroll
+            for (int r = 0; r < 32; ++r)
+                c[r] = Real(0);
+            const int u = lane / VEC, o = lane % VEC;
+#pragma unroll 1
+            for (int I = 0; I < t; ++I, M += 1024)
+#pragma unroll
+                for (int r = 0; r < 32; ++r)
+                    c[r] = fma(M[r * 32 + (u ^ (r & (UNITS - 1))) * VEC + o], xs[32 * I + r], c[r]);
+            Real y;
+            {
+                const Real *xj = xs + 32 * t;
+                const int own = lane * (lane + 1) / 2;
+                Real a0 = 0, a1 = 0;
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                {
+                    const Real v = M[j >= lane ? j * (j + 1) / 2 + lane : own + j];
+                    const Real x = xj[j];
+                    if (j & 1)
+                        a1 = fma(j >= lane ? v : Real(0), x, a1);
+                    else
+                        a0 = fma(j >= lane ? v : Real(0), x, a0);
+                    c[j] = fma(j < lane ? v : Real(0), x, c[j]);
+                }
+#pragma unroll
+                for (int s = 16; s >= 1; s >>= 1)
+#pragma unroll
+                    for (int i = 0; i < s; ++i)
+                        c[i] += c[i + s];
+                y = (a0 + a1) + c[0];
+            }
+            M += 528 + t * 1024; // tile (t, t + 1)
+#pragma unroll 1
+            for (int J = t + 1; J < T; ++J)
+            {
+                const Real *xj = xs + 32 * J;
+                Real a[4] = {Real(0), Real(0), Real(0), Real(0)};
+#pragma unroll
+                for (int q = 0; q < UNITS; ++q)
+                {
+                    const Real *p = M + lane * 32 + (q ^ (lane & (UNITS - 1))) * VEC;
+                    if constexpr (VEC == 2)
+                    {
+                        const double2 v = *reinterpret_cast<const double2 *>(p);
+                        const double2 x = *reinterpret_cast<const double2 *>(xj + q * VEC);
+                        a[(q & 1) * 2] = fma(v.x, x.x, a[(q & 1) * 2]);
+                        a[(q & 1) * 2 + 1] = fma(v.y, x.y, a[(q & 1) * 2 + 1]);
+                    }
+                    else
+                    {
+                        const float4 v = *reinterpret_cast<const float4 *>(p);
+                        const float4 x = *reinterpret_cast<const float4 *>(xj + q * VEC);
+                        a[0] = fma(v.x, x.x, a[0]);
+                        a[1] = fma(v.y, x.y, a[1]);
+                        a[2] = fma(v.z, x.z, a[2]);
+                        a[3] = fma(v.w, x.w, a[3]);
+                    }
+                }
+                y += (a[0] + a[1]) + (a[2] + a[3]);
+                M += J * 1024 + 528; // tile (t, J + 1)
+            }
+            return y;
+        }
+
         // Lane l receives sum over lanes of c[l]; c is destroyed. 31 shuffles.
-        template <class Real>
-        __device__ __forceinline__ Real transpose_sum32(Real (&c)[32], int lane)
+        __device__ __forceinline__ float transpose_sum32(float (&c)[32], int lane)
         {
 #pragma unroll
             for (int s = 16; s >= 1; s >>= 1)
@@ -40,43 +120,43 @@ namespace pmas
 #pragma unroll
                 for (int i = 0; i < s; ++i)
                 {
-                    const Real send = upper ? c[i] : c[i + s];
-                    const Real keep = upper ? c[i + s] : c[i];
+                    const float send = upper ? c[i] : c[i + s];
+                    const float keep = upper ? c[i + s] : c[i];
                     c[i] = keep + __shfl_xor_sync(FULL, send, s);
                 }
             }
             return c[0];
         }
 
-        // Column tile J of y = M x for one tile-packed symmetric matrix (shared memory): adds the
+        // Column tile J of y = M x for one tile-packed FP32 symmetric matrix (shared memory): adds the
         // row contributions of tiles (I, J), I <= J, to yr[I] and the transposed contributions
         // (rows of tile J) to yr[J]. Lane l owns rows 32 t + l.
-        template <int T, class Store, class Real = typename StoreTraits<Store>::Real>
-        __device__ __forceinline__ void symv_column(const Store *__restrict__ M, const Real *__restrict__ xs, int lane,
-                                                    int J, Real (&yr)[T])
+        template <int T>
+        __device__ __forceinline__ void symv_column(const float *__restrict__ M, const float *__restrict__ xs, int lane,
+                                                    int J, float (&yr)[T])
         {
             int off = 0;
 #pragma unroll
             for (int jj = 0; jj < T; ++jj)
                 if (jj < J)
                     off += jj * 1024 + 528;
-            Real cy[32];
+            float cy[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-                cy[j] = Real(0);
+                cy[j] = 0.f;
 #pragma unroll
             for (int I = 0; I < T; ++I)
             {
                 if (I >= J)
                     break;
-                const Store *tile = M + off + I * 1024;
-                const Real xI = xs[32 * I + lane];
-                Real a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+                const float *tile = M + off + I * 1024 + lane * 32;
+                const float xI = xs[32 * I + lane];
+                float a0 = 0, a1 = 0, a2 = 0, a3 = 0;
 #pragma unroll
                 for (int j4 = 0; j4 < 8; ++j4)
                 {
-                    const auto v = load4(tile + j4 * 128 + lane * 4);
-                    const auto xv = load4(xs + 32 * J + 4 * j4);
+                    const float4 v = *reinterpret_cast<const float4 *>(tile + (j4 ^ (lane & 7)) * 4);
+                    const float4 xv = *reinterpret_cast<const float4 *>(xs + 32 * J + 4 * j4);
                     a0 = fma(v.x, xv.x, a0);
                     a1 = fma(v.y, xv.y, a1);
                     a2 = fma(v.z, xv.z, a2);
@@ -89,34 +169,34 @@ namespace pmas
                 yr[I] += (a0 + a1) + (a2 + a3);
             }
             // Diagonal tile, upper triangle by columns.
-            const Store *dt = M + off + J * 1024;
-            const Real xJ = xs[32 * J + lane];
-            Real a0 = 0, a1 = 0;
+            const float *dt = M + off + J * 1024;
+            const float xJ = xs[32 * J + lane];
+            float a0 = 0, a1 = 0;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
             {
-                const Real v = (lane <= j) ? (Real)load1(dt + j * (j + 1) / 2 + lane) : Real(0);
-                const Real xj = xs[32 * J + j];
+                const float v = (lane <= j) ? dt[j * (j + 1) / 2 + lane] : 0.f;
+                const float xj = xs[32 * J + j];
                 if (j & 1)
                     a1 = fma(v, xj, a1);
                 else
                     a0 = fma(v, xj, a0);
-                cy[j] = fma((lane < j) ? v : Real(0), xJ, cy[j]);
+                cy[j] = fma((lane < j) ? v : 0.f, xJ, cy[j]);
             }
-            yr[J] += (a0 + a1) + transpose_sum32<Real>(cy, lane);
+            yr[J] += (a0 + a1) + transpose_sum32(cy, lane);
         }
 
         // y = M x by one warp (all column tiles).
-        template <int T, class Store, class Real = typename StoreTraits<Store>::Real>
-        __device__ __forceinline__ void symv_tiles(const Store *__restrict__ M, const Real *__restrict__ xs, int lane,
-                                                   Real (&yr)[T])
+        template <int T>
+        __device__ __forceinline__ void symv_tiles(const float *__restrict__ M, const float *__restrict__ xs, int lane,
+                                                   float (&yr)[T])
         {
 #pragma unroll
             for (int t = 0; t < T; ++t)
-                yr[t] = Real(0);
+                yr[t] = 0.f;
 #pragma unroll
             for (int J = 0; J < T; ++J)
-                symv_column<T, Store>(M, xs, lane, J, yr);
+                symv_column<T>(M, xs, lane, J, yr);
         }
 
         // ---- Binary16 (mma16 layout): warp tensor-core products, m16n8k16, FP32 accumulation. ----
@@ -281,6 +361,9 @@ namespace pmas
             }
         }
 
+        // Shared-memory shape of the streaming apply. A team of warps multiplies one matrix at a time:
+        // one warp per 32 rows in FP64, else one warp. Two stages per team, as many teams as fit, at
+        // most 16.
         template <int BD, class Store>
         struct ApplyLayout
         {
@@ -289,13 +372,17 @@ namespace pmas
             static constexpr bool MMA = StoreTraits<Store>::SCALED; // binary16: mma16 layout
             static constexpr int S = MMA ? (2 * BD) * (2 * BD - 1) / 2 * 256 + 2 * BD * 192 : N * (N + 1) / 2;
             static constexpr int STAGE_BYTES = S * (int)sizeof(Store);
-            // x: Real values, or binary16 hi / lo columns plus the FP32 result rows.
-            static constexpr int XS_BYTES = MMA ? 8 * N : ((N * (int)sizeof(Real)) + 15) / 16 * 16;
-            static constexpr int WARP_BYTES = 2 * STAGE_BYTES + XS_BYTES + 16;
-            static constexpr int SMEM_LIMIT = 232448 - 1024; // leave room for static shared memory
-            static constexpr int W0 = SMEM_LIMIT / WARP_BYTES;
-            static constexpr int WARPS = W0 > 16 ? 16 : W0;
-            static_assert(STAGE_BYTES % 16 == 0, "bulk copies need 16-byte multiples");
+            static constexpr bool ROWS = std::is_same_v<Store, double>;
+            // x and y of FP64; x of FP32; binary16 hi / lo columns plus the FP32 result rows.
+            static constexpr int XS_BYTES = ROWS ? 16 * N : (MMA ? 8 * N : 4 * N);
+            static constexpr int TEAM = ROWS ? BD : 1; // warps per matrix
+            static constexpr int TEAM_BYTES = 2 * STAGE_BYTES + XS_BYTES + 16;
+            static constexpr int SMEM_LIMIT = 232448 - 1536; // leave room for static shared memory
+            static constexpr int FIT = SMEM_LIMIT / TEAM_BYTES;
+            static constexpr int TEAMS = FIT > 16 ? 16 : FIT;
+            static constexpr int WARPS = TEAMS * TEAM;
+            static constexpr int SMEM = TEAMS * TEAM_BYTES;
+            static_assert(STAGE_BYTES % 16 == 0 && XS_BYTES % 16 == 0, "bulk copies need 16-byte multiples");
         };
 
         // Partial dots of the apply, per CTA: r.z0 and r.z0_old over banks with coupled rows, the
@@ -308,20 +395,20 @@ namespace pmas
         // prefetch_first: issue the first two inverse copies before waiting for the predecessor
         // (a chained launch of one system); otherwise a finished solve returns before any copy
         // (the batched launch, where most CTAs may belong to finished systems).
+        //
+        // Both forms below return with part[] the thread's partial dots, or false on a solve that is
+        // already done. This one: FP32 and binary16 inverses, a warp per matrix.
         template <int BD, class Store, int MODE>
-        __device__ __forceinline__ void mas_apply_body(const MasView &mas, const double *__restrict__ r,
-                                                       double *__restrict__ z0, PcgState *st, const ReduceBuf &red,
-                                                       const PcgConfig &cfg, Cta cta, bool prefetch_first)
+        __device__ __forceinline__ bool mas_apply_warps(const MasView &mas, const double *__restrict__ r,
+                                                        double *__restrict__ z0, PcgState *st, const PcgConfig &cfg,
+                                                        Cta cta, double (&part)[APPLY_PARTS])
         {
-            if (!prefetch_first && MODE != 0 && st->done)
-                return;
             using L = ApplyLayout<BD, Store>;
             using Real = typename L::Real;
             constexpr int N = L::N, S = L::S, WARPS = L::WARPS;
-            constexpr int THREADS = WARPS * 32;
             extern __shared__ __align__(128) unsigned char smem[];
             const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-            unsigned char *base = smem + (size_t)w * L::WARP_BYTES;
+            unsigned char *base = smem + (size_t)w * L::TEAM_BYTES;
             Store *stage0 = reinterpret_cast<Store *>(base);
             Store *stage1 = reinterpret_cast<Store *>(base + L::STAGE_BYTES);
             Real *xs = reinterpret_cast<Real *>(base + 2 * L::STAGE_BYTES);
@@ -367,12 +454,8 @@ namespace pmas
                 if (lane == 0)
                     mbar_drain(bar, pending, {0u, 0u});
                 __syncwarp();
-                return;
+                return false;
             }
-            double part[APPLY_PARTS];
-#pragma unroll
-            for (int i = 0; i < APPLY_PARTS; ++i)
-                part[i] = 0.0;
             uint32_t phase0 = 0, phase1 = 0;
             bool ok = true;
             // Input (and binary16 scale) of the current item, prefetched one item ahead.
@@ -458,9 +541,9 @@ namespace pmas
                 if (!ident)
                 {
                     if constexpr (L::MMA)
-                        symv_mma16<BD>(reinterpret_cast<const __half *>(stage), xh, xl, ys, lane, yr);
+                        symv_mma16<BD>(stage, xh, xl, ys, lane, yr);
                     else
-                        symv_tiles<BD, Store>(stage, xs, lane, yr);
+                        symv_tiles<BD>(stage, xs, lane, yr);
                 }
                 __syncwarp();
                 const int mn = m + 2 * total_warps;
@@ -512,11 +595,204 @@ namespace pmas
                     mbar_drain(bar, pending, {phase0, phase1});
                 __syncwarp();
             }
+            return true;
+        }
+
+        // Barrier of the warps of team `team` (named barriers 1, 2, ...).
+        template <int TEAM>
+        __device__ __forceinline__ void team_sync(int team)
+        {
+            if (TEAM == 1)
+                __syncwarp();
+            else
+                asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(TEAM * 32) : "memory");
+        }
+
+        // FP64 inverses: a team of BD warps per matrix, warp t of the team rows 32 t .. 32 t + 31 (a
+        // lane's row needs no sum across lanes); its first warp also brings the input and forms the
+        // dots. At 96 x 96 an SM works on three matrices and has three on their way. One warp per
+        // matrix with transposed sums by shuffles (as FP32 below keeps: 64.6 us at 80^3 against 74.1 us
+        // by rows) took 8,800 cycles per matrix, too long for the copies to keep going: 86.5 us for the
+        // 8,322 matrices of the 61^3 mesh (310 MB), 54.1 us now, 48 us at the measured copy rate.
+        template <int BD, int MODE>
+        __device__ __forceinline__ bool mas_apply_rows(const MasView &mas, const double *__restrict__ r,
+                                                       double *__restrict__ z0, PcgState *st, const PcgConfig &cfg,
+                                                       Cta cta, double (&part)[APPLY_PARTS])
+        {
+            using L = ApplyLayout<BD, double>;
+            constexpr int N = L::N, S = L::S;
+            extern __shared__ __align__(128) unsigned char smem[];
+            __shared__ int team_failed[L::TEAMS];
+            const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const int team = w / BD, t = w - team * BD;
+            unsigned char *base = smem + (size_t)team * L::TEAM_BYTES;
+            double *xs = reinterpret_cast<double *>(base + 2 * L::STAGE_BYTES);
+            double *ys = xs + N;
+            uint64_t *bar = reinterpret_cast<uint64_t *>(base + 2 * L::STAGE_BYTES + L::XS_BYTES);
+            const double *__restrict__ inv = static_cast<const double *>(mas.inv);
+            const int banks = mas.banks;
+            const int items = banks + mas.n_coarse_active;
+            const int total_teams = cta.n * L::TEAMS;
+            const int gt = cta.x * L::TEAMS + team;
+            int *errp = st ? &st->error : nullptr;
+            const bool pr = (MODE == 2) && cfg.polak_ribiere;
+            const bool loader = t == 0 && lane == 0; // issues the team's copies
+            auto mat_of = [&](int m) { return m < banks ? m : banks + mas.coarse_active[m - banks]; };
+            auto in_of = [&](int m) -> const double * {
+                return m < banks ? r + (size_t)m * N : mas.rc + (size_t)(mat_of(m) - banks) * N;
+            };
+
+            const uint64_t pol = l2_evict_first_policy(); // the inverses stream, the vectors stay
+            bool pending[2] = {gt < items, gt + total_teams < items}; // copies issued and not consumed
+            if (loader)
+            {
+                team_failed[team] = 0;
+                mbar_init(&bar[0], 1);
+                mbar_init(&bar[1], 1);
+                fence_mbar_init();
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+                    if (pending[s])
+                        bulk_load_stream(base + s * L::STAGE_BYTES, inv + (size_t)mat_of(gt + s * total_teams) * S,
+                                         L::STAGE_BYTES, &bar[s], pol);
+            }
+            team_sync<BD>(team);
+            // The first two inverses are on their way (no kernel of a solve writes them); now wait
+            // for the predecessor (launched chained in a PCG iteration).
+            pdl_wait();
+            if (MODE != 0 && st->done)
+            {
+                if (loader)
+                    mbar_drain(bar, pending, {0u, 0u});
+                return false;
+            }
+            uint32_t phase[2] = {0u, 0u};
+            bool ok = true;
+            double r_next[BD]; // first warp: input of the team's next item
+            if (t == 0 && gt < items)
+            {
+                const double *in = in_of(gt);
+#pragma unroll
+                for (int i = 0; i < BD; ++i)
+                    r_next[i] = in[i * 32 + lane];
+            }
+            for (int m = gt, s = 0; m < items; m += total_teams, s ^= 1)
+            {
+                const bool coarse = m >= banks;
+                const int mat = mat_of(m);
+                double *out = coarse ? mas.zc + (size_t)(mat - banks) * N : z0 + (size_t)m * N;
+                double r64[BD], zold[BD];
+                if (t == 0)
+                {
+#pragma unroll
+                    for (int i = 0; i < BD; ++i)
+                    {
+                        r64[i] = r_next[i];
+                        xs[i * 32 + lane] = r64[i];
+                    }
+                    const int mnext = m + total_teams;
+                    if (mnext < items)
+                    {
+                        const double *in = in_of(mnext);
+#pragma unroll
+                        for (int i = 0; i < BD; ++i)
+                            r_next[i] = in[i * 32 + lane];
+                    }
+                    if (pr)
+#pragma unroll
+                        for (int i = 0; i < BD; ++i)
+                            zold[i] = out[i * 32 + lane];
+                }
+                // Coarse matrices of isolated rows are exactly the identity: z = r, unrounded.
+                const bool ident = coarse && mas.identity[mat - banks];
+                if (!mbar_wait_bounded(&bar[s], s ? phase[1] : phase[0], errp, cfg.wait_limit) && lane == 0)
+                    team_failed[team] = 1;
+                team_sync<BD>(team); // x complete; every warp has seen the copy or given up
+                if (team_failed[team])
+                {
+                    ok = false;
+                    break;
+                }
+                pending[s] = false;
+                if (s)
+                    phase[1] ^= 1u;
+                else
+                    phase[0] ^= 1u;
+                if (!ident)
+                    ys[t * 32 + lane] =
+                        symv_row<BD>(reinterpret_cast<const double *>(base + s * L::STAGE_BYTES), xs, t, lane);
+                team_sync<BD>(team); // y complete; the team is done with the stage and with x
+                const int mn = m + 2 * total_teams;
+                if (mn < items)
+                {
+                    if (loader)
+                    {
+                        fence_proxy_async_smem();
+                        bulk_load_stream(base + s * L::STAGE_BYTES, inv + (size_t)mat_of(mn) * S, L::STAGE_BYTES, &bar[s],
+                                         pol);
+                    }
+                    pending[s] = true;
+                }
+                if (t != 0)
+                    continue;
+                double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+                for (int i = 0; i < BD; ++i)
+                {
+                    const double zv = ident ? r64[i] : ys[i * 32 + lane];
+                    out[i * 32 + lane] = zv;
+                    d0 = fma(zv, r64[i], d0);
+                    if (pr)
+                        d1 = fma(zold[i], r64[i], d1);
+                }
+                // Fixed slots (no dynamic indexing, so part[] stays in registers).
+                if (coarse)
+                {
+                    part[4] += d0;
+                    part[5] += d1;
+                }
+                else if (m >= mas.first_iso_bank)
+                {
+                    part[2] += d0;
+                    part[3] += d1;
+                }
+                else
+                {
+                    part[0] += d0;
+                    part[1] += d1;
+                }
+            }
+            if (!ok && loader)
+                mbar_drain(bar, pending, phase); // the outstanding copies (bounded) before leaving
+            return true;
+        }
+
+        template <int BD, class Store, int MODE>
+        __device__ __forceinline__ void mas_apply_body(const MasView &mas, const double *__restrict__ r,
+                                                       double *__restrict__ z0, PcgState *st, const ReduceBuf &red,
+                                                       const PcgConfig &cfg, Cta cta, bool prefetch_first)
+        {
+            if (!prefetch_first && MODE != 0 && st->done)
+                return;
+            using L = ApplyLayout<BD, Store>;
+            constexpr int THREADS = L::WARPS * 32;
+            double part[APPLY_PARTS];
+#pragma unroll
+            for (int i = 0; i < APPLY_PARTS; ++i)
+                part[i] = 0.0;
+            bool ran;
+            if constexpr (L::ROWS)
+                ran = mas_apply_rows<BD, MODE>(mas, r, z0, st, cfg, cta, part);
+            else
+                ran = mas_apply_warps<BD, Store, MODE>(mas, r, z0, st, cfg, cta, part);
+            if (!ran)
+                return;
             pdl_release(); // this warp's items are done: the successor may start launching
             if (MODE == 0)
                 return;
             double tot[APPLY_PARTS];
-            if (grid_reduce<APPLY_PARTS, THREADS>(part, red.rz_parts, &st->counter[4], tot, cta) && threadIdx.x == 0)
+            if (grid_reduce<APPLY_PARTS, THREADS, L::TEAMS * 32>(part, red.rz_parts, &st->counter[4], tot, cta) &&
+                threadIdx.x == 0)
             {
                 // Isolated rows: z = (1 + L) z0, so their r.z is (1 + L) r.z0 -- r.z0 is in the
                 // level-0 sums, the coarse levels add L r.z0.
@@ -1603,7 +1879,7 @@ namespace pmas
         void prepare_variant()
         {
             using L = ApplyLayout<BD, Store>;
-            const int smem = L::WARPS * L::WARP_BYTES;
+            const int smem = L::SMEM;
             cuda_check(cudaFuncSetAttribute(k_mas_apply<BD, Store, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             smem),
                        "apply smem attribute");
@@ -1626,7 +1902,7 @@ namespace pmas
                                PcgConfig cfg, cudaStream_t s)
         {
             using L = ApplyLayout<BD, Store>;
-            const size_t smem = (size_t)L::WARPS * L::WARP_BYTES;
+            const size_t smem = L::SMEM;
             const int grid = mas_apply_grid(mas);
             if (MODE != 0 && grid > red.capacity)
                 throw Error(ERR_INVALID, "[MAS] reduction scratch too small");
@@ -1711,7 +1987,7 @@ namespace pmas
         return grid > 0 ? grid : 0;
     }
 
-    // At least apply_items_per_warp() items per warp (1 by default: the most CTAs, the lowest
+    // At least apply_items_per_warp() items per warp or team of warps (1 by default: the most CTAs, the lowest
     // latency for a lone solve). In batches of small systems more items per warp measured
     // faster: a warp's two-stage copy pipeline runs past its start-up latency, and fewer SMs are
     // held by one system's apply while other systems' kernels run.
@@ -1721,7 +1997,7 @@ namespace pmas
             using L = ApplyLayout<BD, Store>;
             const int sms = device_sm_count();
             const int items = mas.banks + mas.n_coarse_active;
-            const int per_cta = L::WARPS * apply_items_per_warp();
+            const int per_cta = L::TEAMS * apply_items_per_warp();
             int grid = (items + per_cta - 1) / per_cta;
             if (grid > sms)
                 grid = sms;
@@ -1757,7 +2033,7 @@ namespace pmas
             return;
         dispatch(bd, storage, [&]<int BD, class Store>() {
             using L = ApplyLayout<BD, Store>;
-            const size_t smem = (size_t)L::WARPS * L::WARP_BYTES;
+            const size_t smem = L::SMEM;
             if (mode == 1)
                 launch_chained(chained_launch(), k_mas_apply_batch<BD, Store, 1>, total, L::WARPS * 32, smem, s, v);
             else

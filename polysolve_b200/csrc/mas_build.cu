@@ -542,9 +542,10 @@ namespace pmas
                 if (rem < J * 1024)
                 {
                     const int I = rem >> 10, e = rem & 1023;
-                    const int j4 = e >> 7, l = (e & 127) >> 2, jj = e & 3;
+                    constexpr int VEC = 16 / (int)sizeof(Out);
+                    const int l = e >> 5, q = (e & 31) / VEC;
                     row = 32 * I + l;
-                    cl = 32 * J + 4 * j4 + jj;
+                    cl = 32 * J + (q ^ (l & (32 / VEC - 1))) * VEC + e % VEC;
                 }
                 else
                 {

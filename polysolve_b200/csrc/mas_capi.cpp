@@ -2890,7 +2890,7 @@ extern "C" int mas_get_inverses(const mas_solver *h, double *out, size_t count)
                 for (int j = i; j < N; ++j)
                     out[(size_t)m * S + (size_t)i * N - (size_t)i * (i + 1) / 2 + j] =
                         tp[(size_t)m * Ss +
-                           (storage == STORE_F16 ? mma16_index(bd, i, j) : tile_packed_index(bd, i, j))];
+                           (storage == STORE_F16 ? mma16_index(bd, i, j) : tile_packed_index(storage == STORE_F64 ? 2 : 4, i, j))];
     });
 }
 

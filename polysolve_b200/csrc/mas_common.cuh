@@ -42,9 +42,8 @@ namespace pmas
         cuda_check(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...), "kernel launch");
     }
 
-    // Inverse storage types: the arithmetic type of each and loads of one / four consecutive
-    // stored values converted to it. Binary16 values are read as IEEE bits (the buffers are
-    // uint16_t on the host) and multiplied in FP32.
+    // Inverse storage types and the arithmetic type of each. Binary16 values are IEEE bits (the
+    // buffers are uint16_t on the host), multiplied with FP32 accumulation.
     template <class Store>
     struct StoreTraits;
     template <>
@@ -65,19 +64,6 @@ namespace pmas
         using Real = float;
         static constexpr bool SCALED = true;
     };
-
-    __device__ __forceinline__ double4 load4(const double *p) { return *reinterpret_cast<const double4 *>(p); }
-    __device__ __forceinline__ float4 load4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-    __device__ __forceinline__ float4 load4(const __half *p)
-    {
-        const uint2 u = *reinterpret_cast<const uint2 *>(p);
-        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
-        return make_float4(a.x, a.y, b.x, b.y);
-    }
-    __device__ __forceinline__ double load1(const double *p) { return *p; }
-    __device__ __forceinline__ float load1(const float *p) { return *p; }
-    __device__ __forceinline__ float load1(const __half *p) { return __half2float(*p); }
 
     __device__ __forceinline__ double warp_sum(double v)
     {
@@ -134,8 +120,9 @@ namespace pmas
     // Deterministic grid-wide sum of NV values per CTA: every CTA writes its block sum to
     // partials[cta.x * NV + i]; the last CTA to arrive (atomic ticket) adds the partials in a
     // fixed order. Returns true in the last CTA, with tot[] the totals (valid in all its
-    // threads). Every thread of every CTA must call it.
-    template <int NV, int THREADS>
+    // threads). Every thread of every CTA must call it. FINAL: the threads that add the partials, which
+    // with THREADS > FINAL keeps the order of a smaller CTA (warps without a contribution).
+    template <int NV, int THREADS, int FINAL = THREADS>
     __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double *partials, unsigned *counter, double (&tot)[NV],
                                                 Cta cta)
     {
@@ -174,7 +161,7 @@ namespace pmas
         for (int i = 0; i < NV; ++i)
         {
             s[i] = 0.0;
-            for (int b = threadIdx.x; b < cta.n; b += THREADS)
+            for (int b = threadIdx.x; b < cta.n && threadIdx.x < FINAL; b += FINAL)
                 s[i] += __ldcg(partials + (size_t)b * NV + i);
             s[i] = warp_sum(s[i]);
         }

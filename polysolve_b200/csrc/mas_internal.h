@@ -117,14 +117,17 @@ namespace pmas
     // ---------------------------------------------------------------------------------------
     // Subdomain matrix storage ("tile-packed"): an N x N symmetric matrix, N = 32 * bd, split
     // into bd x bd tiles of 32 x 32. For each column tile J: the off-diagonal tiles (I, J), I < J,
-    // each 1024 values with element (l, j) of the tile at (j / 4) * 128 + l * 4 + j % 4; then the
-    // diagonal tile's upper triangle, column j holding rows 0..j at offset j (j + 1) / 2 + l.
+    // each 1024 values by rows, the 16-byte units of row l (vec = 2 FP64 or 4 FP32 values) in
+    // the order q ^ (l mod 32 / vec); then the diagonal tile's upper triangle, column j holding
+    // rows 0..j at offset j (j + 1) / 2 + l. In shared memory a warp then reads a tile without bank
+    // conflicts along rows (lane = row, 16 bytes each) and along columns (lane = column), and the
+    // diagonal tile's rows too (triangular numbers are distinct modulo a power of two).
     // Total N (N + 1) / 2 values, the same count as the reference's packed upper storage.
     // ---------------------------------------------------------------------------------------
     __host__ __device__ inline int tile_packed_size(int bd) { return 32 * bd * (32 * bd + 1) / 2; }
 
     // Position of element (row, col) of the symmetric matrix in tile-packed storage.
-    __host__ __device__ inline int tile_packed_index(int /*bd*/, int row, int col)
+    __host__ __device__ inline int tile_packed_index(int vec, int row, int col)
     {
         if (row > col)
         {
@@ -137,7 +140,7 @@ namespace pmas
         for (int jj = 0; jj < J; ++jj)
             off += jj * 1024 + 528;
         if (I < J)
-            return off + I * 1024 + (j >> 2) * 128 + l * 4 + (j & 3);
+            return off + I * 1024 + l * 32 + ((j / vec) ^ (l & (32 / vec - 1))) * vec + j % vec;
         return off + J * 1024 + j * (j + 1) / 2 + l;
     }
 
