@@ -38,6 +38,7 @@ CU_SOURCES = [
     "mas_build.cu",
     "mas_apply.cu",
     "mas_pcg.cu",
+    "mas_persist.cu",
     "mas_noalloc.cu",
     "mas_multi.cu",
     "mas_multi16.cu",

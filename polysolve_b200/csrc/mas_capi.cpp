@@ -276,6 +276,25 @@ namespace
     }
 
     std::string g_create_error;
+
+    // One cooperative solve at a time on each device: its CTAs wait for one another, so two of them
+    // must not hold parts of the device each. A thread that finds the device taken uses the iteration
+    // kernels (the same bits), as it would overlap with the other solve's kernels anyway.
+    struct CooperativeTurn
+    {
+        static std::atomic<bool> taken[64];
+        int device;
+        bool mine;
+        explicit CooperativeTurn(int dev) : device(dev), mine(dev >= 0 && dev < 64 && !taken[dev].exchange(true)) {}
+        CooperativeTurn(const CooperativeTurn &) = delete;
+        CooperativeTurn &operator=(const CooperativeTurn &) = delete;
+        ~CooperativeTurn()
+        {
+            if (mine)
+                taken[device].store(false);
+        }
+    };
+    std::atomic<bool> CooperativeTurn::taken[64];
 } // namespace
 
 struct mas_solver
@@ -348,6 +367,12 @@ struct mas_solver
     DevBuf<PcgState> st;
     DevBuf<double> partials;
     int red_capacity = 0;
+    // The one-launch solve of small systems (mas_persist.cu): its dots and barrier counter, allocated
+    // with the other vectors when the system is small enough.
+    DevBuf<double> persist_dots, persist_gather;
+    DevBuf<unsigned> persist_bar;
+    bool persist_ready = false;
+    bool in_batch = false; // solving as one of several systems of mas_solve_batch
 
     // Several right-hand sides at once: groups of RHS_GROUP interleaved vectors, one PcgState
     // per right-hand side plus the group record, their own graphs.
@@ -810,6 +835,15 @@ struct mas_solver
         st.alloc(1, "device_buffers scalars");
         red_capacity = std::max({(banks + 7) / 8, mas.total_coarse, device_sm_count() * 8}) + 160;
         partials.alloc((size_t)red_capacity * 9, "device_buffers reduction");
+        persist_ready = banks <= PERSIST_MAX_BANKS && prepare_persistent(bd_, p.storage);
+        if (persist_ready)
+        {
+            persist_dots.alloc(3 * (size_t)((banks + 7) & ~7) + 3 * (size_t)device_sm_count() * 16 + 2,
+                               "device_buffers reduction");
+            persist_gather.alloc(persist_gather_size(mas.view()), "device_buffers p");
+            persist_bar.alloc(1, "device_buffers reduction");
+            cuda_check(cudaMemsetAsync(persist_dots.get(), 0, persist_dots.bytes(), stream), "memset");
+        }
         cuda_check(cudaMemsetAsync(x.get(), 0, x.bytes(), stream), "memset");
         cuda_check(cudaMemsetAsync(pv.get(), 0, pv.bytes(), stream), "memset");
         cuda_check(cudaMemsetAsync(z.get(), 0, z.bytes(), stream), "memset");
@@ -948,13 +982,42 @@ struct mas_solver
         graph_key = key;
     }
 
+    // The shape of the one-launch solve, or one that is not ok: the iteration kernels run instead for
+    // larger systems, Polak-Ribiere (its r.z_old dots), per-kernel profiling, host-launched iterations
+    // (cuda_graphs off) and in batches, where other systems' kernels fill the device.
+    PersistPlan persistent_plan(const MasView &mv, const PcgConfig &cfg) const
+    {
+        PersistPlan pl;
+        if (persist_ready && p.graphs && !p.profile && !in_batch && !cfg.polak_ribiere && p.max_iter >= 1)
+            pl = persist_plan(mv);
+        if (pl.ok && persist_dots_size(mv, pl) > persist_dots.n)
+            pl.ok = false;
+        return pl;
+    }
+
+    // The whole solve in one launch (a long one in slices, so that no launch runs for seconds); the
+    // caller reads h_st[0] after its synchronisation.
+    void pcg_persistent(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, const PersistPlan &pl)
+    {
+        constexpr int SLICE = 2048;
+        PcgState *S = st.get();
+        for (int k0 = 0; k0 == 0 || (k0 < p.max_iter && !h_st[0].done); k0 += SLICE)
+        {
+            run("pcg_persistent", 1, [&] {
+                launch_pcg_persistent(Av, mv, cfg, pl, S, x.get(), r.get(), persist_gather.get(), b.get(),
+                                      persist_dots.get(), persist_bar.get(), k0 == 0 ? 1 : 0, SLICE, p.true_residual_period, stream);
+            });
+            cuda_check(cudaMemcpyAsync(&h_st[0], S, sizeof(PcgState), cudaMemcpyDeviceToHost, stream), "state");
+            cuda_check(cudaStreamSynchronize(stream), "pcg");
+        }
+    }
+
     // pcg_solve (MASSolver.cu:469-595) on device-resident b_ / x_ (padded order).
     void pcg()
     {
         const BankedView Av = A.view();
         const MasView mv = mas.view();
         const PcgConfig cfg = config();
-        PcgState *S = st.get();
         cudaEvent_t e0, e1;
         cuda_check(cudaEventCreate(&e0), "event");
         cuda_check(cudaEventCreate(&e1), "event");
@@ -967,14 +1030,16 @@ struct mas_solver
         set_chained_launch(p.chained);
         set_spmv_unroll(p.spmv_unroll);
         set_apply_items_per_warp(p.apply_ipw);
-        launch_pcg_init_state(S, stream);
-        // r = b - A x, rr0, the level-0 restriction of r, then z = M^-1 r
-        run("spmv_residual", 1, [&] { launch_spmv(SPMV_RESIDUAL, Av, x.get(), r.get(), b.get(), S, red(), 0, 0, stream); });
-        run("restrict", 0, [&] { return launch_restrict(mv, r.get(), S, 0, stream); });
-        apply_levels(mv, cfg, 1);
-        run("update_p", 1, [&] { launch_update_p(mv, x.get(), pv.get(), z.get(), S, 1, stream); });
-        cuda_check(cudaMemcpyAsync(&h_st[0], S, sizeof(PcgState), cudaMemcpyDeviceToHost, stream), "state");
-        cuda_check(cudaStreamSynchronize(stream), "pcg init");
+        PersistPlan pl = persistent_plan(mv, cfg);
+        if (pl.ok)
+        {
+            CooperativeTurn turn(device);
+            pl.ok = turn.mine;
+            if (pl.ok)
+                pcg_persistent(Av, mv, cfg, pl); // returns when the launch has finished
+        }
+        if (!pl.ok)
+            pcg_start(Av, mv, cfg);
         rz0 = h_st[0].rz0;
         rr0 = h_st[0].rr0;
         if (h_st[0].error == ERR_TIMEOUT)
@@ -990,6 +1055,52 @@ struct mas_solver
             throw Error(ERR_NONFINITE, "[MAS] Invalid initial residual.");
         }
         status = MAS_STATUS_RUNNING;
+        if (pl.ok)
+        {
+            cuda_check(cudaEventRecord(e1, stream), "event");
+            cuda_check(cudaEventSynchronize(e1), "pcg");
+            launched_iterations = h_st[0].iter;
+        }
+        else
+            launched_iterations = pcg_iterate(Av, mv, cfg, e1);
+        collect_profile();
+        ev_origin = nullptr;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, e0, e1);
+        solve_ms = ms;
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        const PcgState &f = h_st[0];
+        if (f.error == ERR_TIMEOUT)
+            throw Error(ERR_TIMEOUT, "[MAS] a device-side wait timed out.");
+        if (p.max_iter >= 1)
+            iterations = f.iter;
+        residual_norm = f.res_norm;
+        status = f.status;
+        if (p.max_iter < 1 && iterations == p.max_iter)
+            status = MAS_STATUS_REACH_MAX_ITERATIONS;
+    }
+
+    // The start of a solve by the iteration kernels; h_st[0] holds the state afterwards.
+    void pcg_start(const BankedView &Av, const MasView &mv, const PcgConfig &cfg)
+    {
+        PcgState *S = st.get();
+        launch_pcg_init_state(S, stream);
+        // r = b - A x, rr0, the level-0 restriction of r, then z = M^-1 r
+        run("spmv_residual", 1, [&] { launch_spmv(SPMV_RESIDUAL, Av, x.get(), r.get(), b.get(), S, red(), 0, 0, stream); });
+        run("restrict", 0, [&] { return launch_restrict(mv, r.get(), S, 0, stream); });
+        apply_levels(mv, cfg, 1);
+        run("update_p", 1, [&] { launch_update_p(mv, x.get(), pv.get(), z.get(), S, 1, stream); });
+        cuda_check(cudaMemcpyAsync(&h_st[0], S, sizeof(PcgState), cudaMemcpyDeviceToHost, stream), "state");
+        cuda_check(cudaStreamSynchronize(stream), "pcg init");
+    }
+
+    // The iterations of a solve by the iteration kernels, in chunks of poll_period, until a chunk's
+    // state says done; records e1 after the last one. Returns the iterations launched; h_st[0] holds
+    // the final state.
+    int pcg_iterate(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, cudaEvent_t e1)
+    {
+        PcgState *S = st.get();
         const int P = p.true_residual_period;
         const int chunk = p.poll_period;
         const bool graphs = p.graphs && !p.profile;
@@ -1034,25 +1145,9 @@ struct mas_solver
         cuda_check(cudaEventRecord(e1, stream), "event");
         cuda_check(cudaMemcpyAsync(&h_st[0], S, sizeof(PcgState), cudaMemcpyDeviceToHost, stream), "state");
         cuda_check(cudaStreamSynchronize(stream), "pcg");
-        collect_profile();
-        ev_origin = nullptr;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        solve_ms = ms;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
         cudaEventDestroy(chunk_ev[0]);
         cudaEventDestroy(chunk_ev[1]);
-        launched_iterations = launched;
-        const PcgState &f = h_st[0];
-        if (f.error == ERR_TIMEOUT)
-            throw Error(ERR_TIMEOUT, "[MAS] a device-side wait timed out.");
-        if (p.max_iter >= 1)
-            iterations = f.iter;
-        residual_norm = f.res_norm;
-        status = f.status;
-        if (p.max_iter < 1 && iterations == p.max_iter)
-            status = MAS_STATUS_REACH_MAX_ITERATIONS;
+        return launched;
     }
 
     void load_rhs_device(const double *d_src_b, const double *d_src_x)
@@ -2675,12 +2770,14 @@ extern "C" int mas_solve_batch(mas_solver *const *handles, int count, const doub
     if (!fused)
         parallel_for(count, workers, [&](int i) {
             mas_solver *h = handles[i];
+            h->in_batch = count > 1;
             rc[(size_t)i] = guarded(h, [&] {
                 if (device_pointers)
                     h->solve_device(b[i], x[i], n[i]);
                 else
                     h->solve(b[i], x[i], n[i]);
             });
+            h->in_batch = false;
         });
     int first = MAS_OK;
     for (int i = 0; i < count; ++i)

@@ -568,6 +568,26 @@ namespace pmas
     // Same pattern, new values: re-assemble and re-invert only (the coarse space is kept).
     void refresh_mas_values(MasDevice &M, const BankedMatrix &A, const int *d_node_real, int storage, cudaStream_t s);
 
+    // mas_persist.cu: a whole single-right-hand-side solve in one launch, for small systems. The plan
+    // says whether the system fits (ok) and the launch shape; dots: persist_dots_size doubles, zeroed
+    // once after a factorization; gather: persist_gather_size doubles (p and x as the SpMV gathers
+    // them; kept between the launches of one solve); bar: one counter. first: start the solve, otherwise go on where the
+    // launch before stopped; at most `iters` iterations per launch.
+    constexpr int PERSIST_MAX_BANKS = 4096;
+    struct PersistPlan
+    {
+        bool ok = false;
+        int grid = 0, vgrid = 0, teams = 0, busy = 0, max_items = 0, a_bytes = 0, deep_nodes = 0, staged = 0;
+        size_t smem = 0;
+    };
+    bool prepare_persistent(int bd, int storage); // false: no cooperative launch of this shape here
+    PersistPlan persist_plan(const MasView &mas);
+    size_t persist_dots_size(const MasView &mas, const PersistPlan &pl);
+    size_t persist_gather_size(const MasView &mas);
+    void launch_pcg_persistent(const BankedView &A, const MasView &mas, const PcgConfig &cfg, const PersistPlan &pl,
+                               PcgState *st, double *x, double *r, double *gather, const double *b, double *dots,
+                               unsigned *bar, int first, int iters, int period, cudaStream_t s);
+
     // mas_pcg.cu: misc
     void launch_zero(double *p, size_t n, cudaStream_t s);
 

@@ -1,0 +1,1012 @@
+// The whole PCG solve of one system in one launch (sm_100a), for systems whose subdomain inverses fit
+// in the shared memory of all SMs. The iteration kernels of such a system are bound by latency:
+// launch, first loads and grid reduction, five times per iteration.
+//
+// Every CTA (one per SM) owns a fixed set of work items for the whole solve: MAS subdomains (banks,
+// with their 32 block rows of the matrix and of x, r, p) and coarse matrices. It keeps in shared
+// memory the vectors of its rows, its inverses and as many of its matrix rows as fit. Only p
+// (gathered by the SpMV), the coarse vectors and the dot products pass through global memory, so an
+// iteration is four grid barriers:
+//
+//   y = A p, p.y  | A |  r -= alpha y, r.r, level-0 restriction | B |  coarse sums and matrices | C |
+//   beta, x += alpha p, p = z + beta p  | D |
+//
+// and the level-0 inverses are applied between the arrival at barrier B and the wait. On iterations
+// that recompute the true residual a fifth barrier follows the update of x.
+//
+// The arithmetic and its order are those of the iteration kernels, so the iterates have the same bits:
+// every per-bank dot is the warp sum the kernels form, and the totals are added in the order of their
+// two-stage reductions (8 banks per CTA for p.Ap and r.r; the apply's teams -- item m belongs to
+// team m mod (grid * teams per CTA) -- for r.z). Each CTA computes all totals and the scalar step
+// itself.
+//
+// Measured (solve_device, us per solve, iteration kernels -> one launch): 20^3 elasticity FP16 1,870 ->
+// 955 (17 us per iteration), 33^3 FP16 3,060 -> 2,150, 200 x 100 plane FP16 3,850 -> 2,160, 30^3
+// scalar FP64 3,040 -> 1,720, 8^3 FP64 1,240 -> 640. An iteration at 20^3 is some 30,000 cycles: four
+// barriers of 2,400 (148 CTAs), 8,500 for the slowest CTA's SpMV (two rounds of gathers from L2), 4,000
+// for the totals and the scalar step, 7,000 for the coarse levels.
+
+#include "mas_apply.cuh"
+
+namespace pmas
+{
+    namespace
+    {
+        constexpr int PS_THREADS = 384;
+        constexpr int PS_WARPS = PS_THREADS / 32;
+        constexpr unsigned PS_ABORT = 0x80000000u;
+        // Polls of a grid barrier before the solve gives up (some seconds).
+        constexpr int PS_SPIN_LIMIT = 1 << 22;
+
+        // Per-warp scratch of the apply: the binary16 hi / lo input and 32 result rows, or the FP32 input.
+        template <int BD, class Store>
+        constexpr size_t PS_SCRATCH = StoreTraits<Store>::SCALED ? 128 * BD + 128
+                                                                 : (std::is_same_v<Store, float> ? 128 * BD : 0);
+
+        struct PersistArgs
+        {
+            BankedView A;
+            MasView mas;
+            PcgConfig cfg;
+            PcgState *st;
+            double *x, *r;
+            double *pg, *xg; // p, and x of the last true residual, as the SpMV gathers them
+            const double *b;
+            double *dots;  // per-bank and per-team dots (persist_dots_size)
+            unsigned *bar; // arrivals at the grid barriers of this launch (zero at the start)
+            int items;     // banks + active coarse matrices
+            int teams;     // teams of the apply: its grid * its teams per CTA
+            int vgrid;     // the apply's grid
+            int busy;      // teams with work
+            int max_items; // most items of a CTA
+            int a_bytes;   // shared memory for matrix rows (and the lists of the coarse sums)
+            int deep_nodes; // nodes of the coarse levels above the first
+            int staged;     // dots staged at a time
+            int first;      // start the solve (otherwise go on from st, x, r, p)
+            int iters;      // iterations of this launch at most
+            int period;     // true-residual period (0: never)
+        };
+
+        // Shared-memory record of one work item. Coarse matrices use r (input) and yz (output) only.
+        template <int BD>
+        struct alignas(16) ItemRec
+        {
+            double x[32 * BD], r[32 * BD], p[32 * BD];
+            double yz[32 * BD]; // A p, then z
+            int4 cslot[32];
+            int key[32], len[32];
+            const double *avals; // matrix rows: values and columns (shared memory if resident)
+            const int *acols;
+            double scale;
+            int m, mat;      // work item and matrix
+            int ident;       // the inverse is exactly the identity
+            int resident;
+            int width, base; // bank: slots per row, first component; coarse matrix above the first level:
+                             // end of its level in `deep`, and the offset of a coarse node there
+        };
+
+        struct PsShared
+        {
+            PcgState st;
+            double red[16];
+            double tot[3];
+            uint64_t bar;
+            int deep_top, deep_lo, deep_hi; // coarse levels above the first: highest level this CTA needs,
+                                            // its range of level-1 nodes
+        };
+
+        __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p)
+        {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+            return v;
+        }
+
+        __device__ __forceinline__ void red_release_gpu(unsigned *p, unsigned v)
+        {
+            asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+        }
+
+        // Grid barrier: arrive, then wait. Monotonic arrival count (no reset inside a launch); the top
+        // bit tells every CTA that one gave up. A wait that runs out sets it too.
+        __device__ __forceinline__ void ps_arrive(unsigned *bar)
+        {
+            __syncthreads();
+            if (threadIdx.x == 0)
+                red_release_gpu(bar, 1u);
+        }
+
+        __device__ __forceinline__ bool ps_wait(unsigned *bar, unsigned &target)
+        {
+            target += gridDim.x;
+            bool gave_up = false;
+            if (threadIdx.x == 0)
+            {
+                unsigned v = 0;
+#pragma unroll 1
+                for (int i = 0; i < PS_SPIN_LIMIT && v < target; ++i)
+                    v = ld_acquire_gpu(bar); // the abort bit ends the wait too
+                gave_up = v < target || (v & PS_ABORT);
+                if (gave_up)
+                    atomicOr(bar, PS_ABORT);
+            }
+            return !__syncthreads_or(gave_up);
+        }
+
+        __device__ __forceinline__ bool ps_barrier(unsigned *bar, unsigned &target)
+        {
+            ps_arrive(bar);
+            return ps_wait(bar, target);
+        }
+
+        // Global dots (written before the last grid barrier) into shared memory, 16 bytes per thread and
+        // step: every CTA reads the same lines at the same time, so the number of requests counts.
+        __device__ __forceinline__ void stage_dots(const double *src, int count, double *dst)
+        {
+            for (int i = threadIdx.x * 2; i < count; i += PS_THREADS * 2)
+                *reinterpret_cast<double2 *>(dst + i) = __ldcg(reinterpret_cast<const double2 *>(src + i));
+        }
+
+        // Sum of staged per-bank dots in the order of the SpMV's and update_xr's two-stage reduction (8
+        // banks per CTA, 256 threads in the last CTA). Every thread must call it; `sh` (8 doubles) holds
+        // the warp sums after the caller's next barrier, bank_total adds them.
+        __device__ __forceinline__ void bank_dots_stage(const double *dots, int banks, double *sh, int w)
+        {
+            if (w >= 8)
+                return;
+            const int groups = (banks + 7) / 8;
+            double s = 0.0;
+            for (int g = threadIdx.x; g < groups; g += 256)
+            {
+                double t = 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    t += dots[g * 8 + i];
+                s += t;
+            }
+            s = warp_sum(s);
+            if ((threadIdx.x & 31) == 0)
+                sh[w] = s;
+        }
+
+        __device__ __forceinline__ double bank_total(const double *sh)
+        {
+            double t = 0.0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w)
+                t += sh[w];
+            return t;
+        }
+
+        // The gathered vectors (p, and x on true-residual iterations) hold a node's values in 32 bytes at
+        // block_dim 3, so that one 32-byte load brings them.
+        template <int BD>
+        constexpr int GATHER_STRIDE = BD == 3 ? 4 : BD;
+
+        template <int BD>
+        __device__ __forceinline__ void gather_node(const double *v, int node, double (&x)[BD])
+        {
+            const double *q = v + node * GATHER_STRIDE<BD>;
+            if constexpr (BD == 3)
+            {
+                double pad;
+                asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];"
+                             : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(pad)
+                             : "l"(q)
+                             : "memory");
+            }
+            else if constexpr (BD == 2)
+            {
+                const double2 t = __ldcg(reinterpret_cast<const double2 *>(q));
+                x[0] = t.x;
+                x[1] = t.y;
+            }
+            else
+                x[0] = __ldcg(q);
+        }
+
+        // One bank's rows of y = A v by one warp (lane = block row). v was written by other CTAs before
+        // the last grid barrier. RES: the rows are in shared memory, so only the gathers of v take
+        // time: U of them in flight. Otherwise everything comes from L2. Slots past a row's end hold
+        // column 0; their products are not added.
+        template <int BD, int U, bool RES>
+        __device__ __forceinline__ void bank_rows(const double *vp, const int *cp, int len, int width, const double *v,
+                                                  int lane, double (&acc)[BD])
+        {
+            constexpr int BS = BD * BD, PAIRS = BS / 2;
+            cp += lane;
+            vp += lane * 2;
+            auto load_block = [&](int k, double(&q)[BS]) {
+                const double *blk = vp + k * 32 * BS;
+#pragma unroll
+                for (int i = 0; i < PAIRS; ++i)
+                {
+                    const double2 *s = reinterpret_cast<const double2 *>(blk + i * 64);
+                    const double2 t = RES ? *s : __ldg(s);
+                    q[2 * i] = t.x;
+                    q[2 * i + 1] = t.y;
+                }
+                if (BS & 1)
+                    q[BS - 1] = RES ? blk[PAIRS * 64 - lane] : __ldg(blk + PAIRS * 64 - lane);
+            };
+            int cn[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                cn[u] = u < width ? (RES ? cp[u * 32] : __ldg(cp + u * 32)) : 0;
+#pragma unroll 1
+            for (int k0 = 0; k0 < width; k0 += U)
+            {
+                double xc[U][BD], m[RES ? 2 : U][BS];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    gather_node<BD>(v, cn[u], xc[u]);
+                if (!RES)
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        load_block(min(k0 + u, width - 1), m[RES ? 0 : u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    cn[u] = k0 + U + u < width ? (RES ? cp[(k0 + U + u) * 32] : __ldg(cp + (k0 + U + u) * 32)) : 0;
+                if (RES)
+                    load_block(k0, m[0]);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    if (RES && u + 1 < U)
+                        load_block(min(k0 + u + 1, width - 1), m[RES ? (u + 1) & 1 : 0]);
+                    const bool in = k0 + u < len;
+#pragma unroll
+                    for (int i = 0; i < BD; ++i)
+#pragma unroll
+                        for (int j = 0; j < BD; ++j)
+                        {
+                            const double t = fma(m[RES ? u & 1 : u][i * BD + j], xc[u][j], acc[i]);
+                            acc[i] = in ? t : acc[i];
+                        }
+                }
+            }
+        }
+
+        // Row 32 t + lane of y = M x for one mma16 matrix in shared memory: block rows 2 t and 2 t + 1 of
+        // symv_mma16, each block row's products in the same order (block columns left to right, then
+        // the diagonal block).
+        template <int BD>
+        __device__ __forceinline__ float symv_mma16_rows(const __half *M, const __half *xh, const __half *xl, float *ys,
+                                                         int t, int lane)
+        {
+            constexpr int NS = 2 * BD, NB = NS * (NS - 1) / 2;
+            const int g = lane >> 2, q = lane & 3;
+            const int c = lane >> 3, rr = lane & 7;
+            const __half *xsrc = (g == 0) ? xh : xl;
+            const uint32_t mbase = smem_addr(M) + (uint32_t)(rr * 16);
+            const int ct = (c == 1) ? 2 : (c == 2 ? 1 : c);
+            const int cd = (c == 1) ? 1 : (c == 3 ? 2 : 0);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+            {
+                const int R = 2 * t + h;
+                float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int i = 0; i < NS; ++i)
+                {
+                    const int S = i < NS - 1 ? (i < R ? i : i + 1) : R; // the diagonal block last
+                    const uint32_t b0 = g < 2 ? *reinterpret_cast<const uint32_t *>(xsrc + 16 * S + 2 * q) : 0u;
+                    const uint32_t b1 = g < 2 ? *reinterpret_cast<const uint32_t *>(xsrc + 16 * S + 2 * q + 8) : 0u;
+                    uint32_t a[4];
+                    if (i == NS - 1)
+                    {
+                        const uint32_t blk = mbase + (uint32_t)((NB * 256 + R * 192) * 2);
+                        ldsm_x4_trans(a, blk + cd * 128);
+                        a[2] = ldsm_x1(blk + 128);
+                    }
+                    else
+                    {
+                        const int lo = S < R ? S : R, hi = S < R ? R : S;
+                        const uint32_t blk = mbase + (uint32_t)((lo * (2 * NS - lo - 1) / 2 + (hi - lo - 1)) * 512);
+                        if (S > R)
+                            ldsm_x4(a, blk + c * 128);
+                        else
+                            ldsm_x4_trans(a, blk + ct * 128);
+                    }
+                    mma_16816(d, a, b0, b1);
+                }
+                if (q == 0)
+                {
+                    ys[16 * h + g] = d[0] + d[1];
+                    ys[16 * h + g + 8] = d[2] + d[3];
+                }
+            }
+            __syncwarp();
+            return ys[lane];
+        }
+
+        template <int BD, class Store>
+        __global__ void __launch_bounds__(PS_THREADS, 1) k_pcg_persistent(const __grid_constant__ PersistArgs a)
+        {
+            using L = ApplyLayout<BD, Store>;
+            using Real = typename L::Real;
+            using Rec = ItemRec<BD>;
+            constexpr int N = L::N, BS = BD * BD;
+            extern __shared__ __align__(128) unsigned char smem[];
+            __shared__ PsShared sh;
+            // The warp index as a broadcast, so that the compiler knows it to be uniform in the warp: in
+            // branches and loops that it cannot prove uniform it guards every shuffle, and a warp sum
+            // takes 2,500 cycles instead of 250.
+            const int tid = threadIdx.x, w = __shfl_sync(FULL, tid >> 5, 0), lane = tid & 31;
+            const MasView &mas = a.mas;
+            const int banks = mas.banks;
+
+            // ---- The CTA's items: teams [v0, v0 + nv), item j = (k, v) in increasing order (item m =
+            // v0 + v + k * teams), so its nb banks come before its coarse matrices.
+            const int v0 = (int)((long long)blockIdx.x * a.busy / gridDim.x);
+            const int nv = (int)((long long)(blockIdx.x + 1) * a.busy / gridDim.x) - v0;
+            int ni = 0, nb = 0;
+#pragma unroll 1
+            for (int k = v0; k < a.items; k += a.teams)
+            {
+                ni += min(nv, a.items - k);
+                nb += max(0, min(nv, banks - k));
+            }
+
+            // ---- Shared memory.
+            Rec *rec = reinterpret_cast<Rec *>(smem);
+            unsigned char *at = smem + (size_t)a.max_items * sizeof(Rec);
+            unsigned char *scratch = at + (size_t)w * PS_SCRATCH<BD, Store>;
+            at += (size_t)PS_WARPS * PS_SCRATCH<BD, Store>;
+            double *vpart = reinterpret_cast<double *>(at); // 3 * vgrid partials of the apply's dots
+            at += (size_t)((3 * a.vgrid + 1) & ~1) * sizeof(double);
+            double *deep = reinterpret_cast<double *>(at); // coarse sums above the first level
+            at += (size_t)((a.deep_nodes * BD + 1) & ~1) * sizeof(double);
+            double *staged = reinterpret_cast<double *>(at); // dots of every CTA
+            at += (size_t)a.staged * sizeof(double);
+            unsigned short *kids = reinterpret_cast<unsigned short *>(at); // children of the nodes of `deep`
+            at += (size_t)a.deep_nodes * 64;
+            unsigned char *slots = at; // the inverses
+            unsigned char *a_rows = slots + (size_t)a.max_items * L::STAGE_BYTES;
+            const unsigned char *inv = static_cast<const unsigned char *>(mas.inv);
+
+            double *dot_pap = a.dots;
+            const int bank_pad = (banks + 7) & ~7;
+            double *dot_bb = a.dots + bank_pad, *dot_rr = a.dots + 2 * bank_pad, *dot_rz = a.dots + 3 * bank_pad;
+
+            // ---- Load the CTA's part of the system.
+            if (tid == 0)
+            {
+                sh.deep_top = sh.deep_lo = sh.deep_hi = 0;
+                mbar_init(&sh.bar, 1);
+                fence_mbar_init();
+                unsigned *z = reinterpret_cast<unsigned *>(&sh.st);
+                const unsigned *src = reinterpret_cast<const unsigned *>(a.st);
+#pragma unroll 1
+                for (int i = 0; i < (int)(sizeof(PcgState) / sizeof(unsigned)); ++i)
+                    z[i] = a.first ? 0u : src[i];
+            }
+#pragma unroll 1
+            for (int j = w; j < ni; j += PS_WARPS)
+            {
+                Rec &it = rec[j];
+                const int m = v0 + j % nv + (j / nv) * a.teams;
+                if (lane == 0)
+                {
+                    it.m = m;
+                    it.mat = m < banks ? m : banks + mas.coarse_active[m - banks];
+                    it.scale = StoreTraits<Store>::SCALED ? mas.inv_scale[it.mat] : 1.0;
+                    it.ident = m >= banks ? mas.identity[it.mat - banks] : 0;
+                }
+                if (m >= banks)
+                    continue;
+                it.len[lane] = a.A.rowlen[m * 32 + lane];
+                it.key[lane] = m < mas.first_iso_bank ? mas.lcco0[m * 32 + lane] : -1;
+                it.cslot[lane] = mas.cslot[m * 32 + lane];
+#pragma unroll 1
+                for (int e = lane; e < N; e += 32)
+                {
+                    const size_t q = (size_t)m * N + e;
+                    const size_t g = (size_t)(m * 32 + e / BD) * GATHER_STRIDE<BD> + e % BD;
+                    it.x[e] = a.x[q];
+                    it.p[e] = a.first ? 0.0 : a.pg[g];
+                    it.r[e] = a.first ? 0.0 : a.r[q];
+                    a.xg[g] = it.x[e];
+                }
+                if (lane == 0)
+                {
+                    const long long s0 = a.A.slice[m];
+                    it.width = (int)(a.A.slice[m + 1] - s0);
+                    it.base = m < mas.first_iso_bank ? mas.cco0_base[m] : 0;
+                    it.avals = a.A.vals + s0 * 32 * BS;
+                    it.acols = a.A.cols + s0 * 32;
+                    it.resident = 0;
+                }
+            }
+            __syncthreads();
+            if (tid == 0)
+            {
+                // The inverses, and the matrix rows that fit, by bulk copies on one barrier.
+                int used = 0;
+#pragma unroll 1
+                for (int j = 0; j < nb; ++j)
+                {
+                    const int bytes = rec[j].width * 32 * (BS * 8 + 4);
+                    if (bytes > 0 && used + bytes <= a.a_bytes)
+                    {
+                        rec[j].resident = 1;
+                        used += bytes;
+                    }
+                }
+                mbar_arrive_expect_tx(&sh.bar, (uint32_t)(used + ni * L::STAGE_BYTES));
+                used = 0;
+#pragma unroll 1
+                for (int j = 0; j < ni; ++j)
+                {
+                    bulk_copy_g2s(slots + (size_t)j * L::STAGE_BYTES, inv + (size_t)rec[j].mat * L::STAGE_BYTES,
+                                  L::STAGE_BYTES, &sh.bar);
+                    if (j >= nb || !rec[j].resident)
+                        continue;
+                    const uint32_t vb = (uint32_t)rec[j].width * 32 * BS * 8, cb = (uint32_t)rec[j].width * 32 * 4;
+                    bulk_copy_g2s(a_rows + used, rec[j].avals, vb, &sh.bar);
+                    bulk_copy_g2s(a_rows + used + vb, rec[j].acols, cb, &sh.bar);
+                    rec[j].avals = reinterpret_cast<const double *>(a_rows + used);
+                    rec[j].acols = reinterpret_cast<const int *>(a_rows + used + vb);
+                    used += vb + cb;
+                }
+                // The coarse sums above the first level that this CTA's coarse matrices take.
+#pragma unroll 1
+                for (int j = nb; j < ni; ++j)
+                {
+                    const int g0 = (rec[j].mat - banks) * 32; // first coarse node of the matrix
+                    int l = 0, below = 0;                     // its level, and the level's first node in `deep`
+#pragma unroll 1
+                    while (l + 1 < mas.level_num && g0 >= mas.coff[l + 1])
+                    {
+                        below += l > 0 ? mas.real_count[l] : 0;
+                        ++l;
+                    }
+                    rec[j].base = l > 0 ? below - mas.coff[l] : 0;
+                    rec[j].width = l > 0 ? below + mas.real_count[l] : 0;
+                    if (l > 0)
+                    {
+                        const int f = l == 1 ? g0 - mas.coff[1] : 0;
+                        const int e = l == 1 ? min(f + 32, mas.real_count[1]) : mas.real_count[1];
+                        sh.deep_lo = sh.deep_top == 0 ? f : min(sh.deep_lo, f);
+                        sh.deep_hi = max(sh.deep_hi, e);
+                        sh.deep_top = max(sh.deep_top, l);
+                    }
+                }
+            }
+            __syncthreads();
+            // Without its inverses and rows the CTA must not go on: it tells the others and leaves.
+            bool ok = __syncthreads_and(mbar_wait_bounded(&sh.bar, 0u, nullptr, a.cfg.wait_limit)) != 0;
+            if (!ok && tid == 0)
+                atomicOr(a.bar, PS_ABORT);
+            unsigned target = 0;
+            const int deep_top = __shfl_sync(FULL, sh.deep_top, 0), deep_lo = __shfl_sync(FULL, sh.deep_lo, 0),
+                      deep_hi = __shfl_sync(FULL, sh.deep_hi, 0);
+            {
+                int to = 0; // the level's first node
+#pragma unroll 1
+                for (int l = 1; l <= deep_top; to += mas.real_count[l], ++l)
+#pragma unroll 1
+                    for (int i = (l == 1 ? deep_lo : 0) + w; i < (l == 1 ? deep_hi : mas.real_count[l]); i += PS_WARPS)
+                    {
+                        const int kb = mas.kid_ptr[l][i], ke = mas.kid_ptr[l][i + 1];
+                        kids[(to + i) * 32 + lane] = kb + lane < ke ? (unsigned short)mas.kids[kb + lane] : 0xFFFF;
+                    }
+            }
+            // x is where the first residual gathers it once every CTA is past this barrier (which also
+            // orders the table above).
+            ok = ps_barrier(a.bar, target) && ok;
+
+#pragma unroll 1
+            for (int n = a.first ? -1 : 0; ok; ++n)
+            {
+                const bool init = n < 0;
+                // ---- y = A p and p.y, or (start, and true-residual iterations after their x update)
+                // r = b - A x with r.r.
+                bool residual = init;
+#pragma unroll 1
+                for (;;)
+                {
+                    const double *v = residual ? a.xg : a.pg;
+#pragma unroll 1
+                    for (int j = w; j < nb; j += PS_WARPS)
+                    {
+                        Rec &it = rec[j];
+                        double acc[BD], part = 0.0, bb = 0.0;
+#pragma unroll
+                        for (int i = 0; i < BD; ++i)
+                            acc[i] = 0.0;
+                        if (__shfl_sync(FULL, it.resident, 0))
+                            bank_rows<BD, 8, true>(it.avals, it.acols, it.len[lane], __shfl_sync(FULL, it.width, 0), v, lane, acc);
+                        else
+                            bank_rows<BD, BD == 3 ? 3 : 4, false>(it.avals, it.acols, it.len[lane], __shfl_sync(FULL, it.width, 0), v, lane, acc);
+#pragma unroll
+                        for (int i = 0; i < BD; ++i)
+                        {
+                            const int e = lane * BD + i;
+                            if (residual)
+                            {
+                                const double bv = a.b[(size_t)it.m * N + e];
+                                acc[i] = bv - acc[i];
+                                it.r[e] = acc[i];
+                                bb = fma(bv, bv, bb);
+                            }
+                            else
+                                it.yz[e] = acc[i];
+                            part = fma(acc[i], residual ? acc[i] : it.p[e], part);
+                        }
+                        part = warp_sum(part);
+                        if (init)
+                            bb = warp_sum(bb);
+                        if (lane == 0)
+                        {
+                            (residual ? dot_rr : dot_pap)[it.m] = part;
+                            if (init)
+                                dot_bb[it.m] = bb;
+                        }
+                    }
+                    if (residual)
+                        break;
+                    if (!(ok = ps_barrier(a.bar, target)))
+                        break;
+                    stage_dots(dot_pap, bank_pad, staged);
+                    __syncthreads();
+                    bank_dots_stage(staged, banks, sh.red, w);
+                    __syncthreads();
+                    const double pap = bank_total(sh.red);
+                    const double alpha = (fabs(pap) < 1e-20) ? 0.0 : sh.st.rz / pap;
+                    residual = a.period > 0 && (__shfl_sync(FULL, sh.st.iter, 0) + 1) % a.period == 0;
+                    if (tid == 0)
+                    {
+                        sh.st.pAp = pap;
+                        sh.st.alpha = alpha;
+                    }
+#pragma unroll 1
+                    for (int j = w; j < nb; j += PS_WARPS)
+                    {
+                        Rec &it = rec[j];
+                        double part = 0.0;
+#pragma unroll
+                        for (int t = 0; t < BD; ++t)
+                        {
+                            const int e = t * 32 + lane;
+                            if (residual)
+                            {
+                                const double xn = fma(alpha, it.p[e], it.x[e]);
+                                it.x[e] = xn;
+                                a.xg[(it.m * 32 + e / BD) * GATHER_STRIDE<BD> + e % BD] = xn;
+                            }
+                            else
+                            {
+                                const double rv = fma(-alpha, it.yz[e], it.r[e]);
+                                it.r[e] = rv;
+                                part = fma(rv, rv, part);
+                            }
+                        }
+                        if (residual)
+                            continue;
+                        part = warp_sum(part);
+                        if (lane == 0)
+                            dot_rr[it.m] = part;
+                    }
+                    if (!residual)
+                        break;
+                    if (!(ok = ps_barrier(a.bar, target)))
+                        break;
+                }
+                if (!ok)
+                    break;
+                // ---- Level-0 restriction of r (a warp's own banks).
+                __syncwarp();
+#pragma unroll 1
+                for (int j = w; j < nb; j += PS_WARPS)
+                {
+                    Rec &it = rec[j];
+                    if (__shfl_sync(FULL, it.m, 0) >= mas.first_iso_bank)
+                        continue;
+                    double rv[BD];
+#pragma unroll
+                    for (int i = 0; i < BD; ++i)
+                        rv[i] = it.r[lane * BD + i];
+                    warp_segment_store<BD>(rv, it.key[lane], it.base, mas.rc);
+                }
+                ps_arrive(a.bar);
+
+                // ---- The MAS apply, 32 rows of one matrix per warp. The subdomain matrices need this CTA's
+                // r only; the coarse ones every CTA's.
+#pragma unroll 1
+                for (int part = 0; part < 2; ++part)
+                {
+                    if (part == 1)
+                    {
+                        if (!(ok = ps_wait(a.bar, target)) || nb == ni)
+                            break;
+                        // Coarse levels above the first: a warp per node, lane = child (the order of
+                        // k_coarse_levels), two nodes at a time.
+                        int from = 0, to = 0; // first node of the level below and of the level
+#pragma unroll 1
+                        for (int l = 1; l <= deep_top; ++l)
+                        {
+                            const int hi = l == 1 ? deep_hi : mas.real_count[l];
+#pragma unroll 1
+                            for (int i = (l == 1 ? deep_lo : 0) + w; i < hi; i += 2 * PS_WARPS)
+                            {
+                                double t[2][BD];
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+                                {
+                                    const int kid = i + h * PS_WARPS < hi ? kids[(to + i + h * PS_WARPS) * 32 + lane] : 0xFFFF;
+#pragma unroll
+                                    for (int c = 0; c < BD; ++c)
+                                    {
+                                        t[h][c] = 0.0;
+                                        if (kid != 0xFFFF)
+                                            t[h][c] = l == 1 ? __ldcg(mas.rc + (mas.coff[0] + kid) * BD + c)
+                                                             : deep[(from + kid) * BD + c];
+                                    }
+                                }
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                                    for (int c = 0; c < BD; ++c)
+                                    {
+                                        t[h][c] = warp_sum(t[h][c]);
+                                        if (lane == 0 && i + h * PS_WARPS < hi)
+                                            deep[(to + i + h * PS_WARPS) * BD + c] = t[h][c];
+                                    }
+                            }
+                            __syncthreads();
+                            from = to;
+                            to += mas.real_count[l];
+                        }
+                        // The coarse inputs.
+#pragma unroll 1
+                        for (int q = tid; q < (ni - nb) * N; q += PS_THREADS)
+                        {
+                            Rec &it = rec[nb + q / N];
+                            const int e = q % N, node = (it.mat - banks) * 32 + e / BD + it.base;
+                            it.r[e] = node < it.width ? deep[node * BD + e % BD]
+                                                      : __ldcg(mas.rc + (size_t)(it.mat - banks) * N + e);
+                        }
+                        __syncthreads();
+                    }
+                    const int j0 = part ? nb : 0, tasks = (part ? ni - nb : nb) * BD;
+#pragma unroll 1
+                    for (int k = w; k < tasks; k += PS_WARPS)
+                    {
+                        const int j = j0 + k / BD, t = k % BD, e = t * 32 + lane;
+                        Rec &it = rec[j];
+                        const Store *M = reinterpret_cast<const Store *>(slots + (size_t)j * L::STAGE_BYTES);
+                        double zv;
+                        if constexpr (L::MMA)
+                        {
+                            __half *xh = reinterpret_cast<__half *>(scratch), *xl = xh + N;
+                            double rv[BD], amax = 0.0;
+#pragma unroll
+                            for (int i = 0; i < BD; ++i)
+                            {
+                                rv[i] = it.r[i * 32 + lane];
+                                amax = fmax(amax, fabs(rv[i]));
+                            }
+#pragma unroll
+                            for (int o = 16; o >= 1; o >>= 1)
+                                amax = fmax(amax, __shfl_xor_sync(FULL, amax, o));
+                            const double xscale = (amax > 0.0 && isfinite(amax)) ? ldexp(1.0, 14 - ilogb(amax)) : 1.0;
+#pragma unroll
+                            for (int i = 0; i < BD; ++i)
+                            {
+                                const float f = (float)(rv[i] * xscale);
+                                const __half h = __float2half_rn(f);
+                                xh[i * 32 + lane] = h;
+                                xl[i * 32 + lane] = __float2half_rn(f - __half2float(h));
+                            }
+                            __syncwarp();
+                            zv = (double)symv_mma16_rows<BD>(M, xh, xl, reinterpret_cast<float *>(xl + N), t, lane) *
+                                 (it.scale / xscale);
+                        }
+                        else if constexpr (std::is_same_v<Real, double>)
+                            zv = symv_row<BD>(M, it.r, t, lane);
+                        else
+                        {
+                            float *xs = reinterpret_cast<float *>(scratch);
+#pragma unroll
+                            for (int i = 0; i < BD; ++i)
+                                xs[i * 32 + lane] = (float)it.r[i * 32 + lane];
+                            __syncwarp();
+                            zv = (double)symv_row<BD>(M, xs, t, lane);
+                        }
+                        if (it.ident)
+                            zv = it.r[e];
+                        it.yz[e] = zv;
+                        if (part == 1)
+                            mas.zc[(size_t)(it.mat - banks) * N + e] = zv;
+                        __syncwarp(); // the scratch is read
+                    }
+                }
+                if (!ok)
+                    break;
+                __syncthreads();
+                // ---- r.z per team: its items in order, then the warp sum.
+#pragma unroll 1
+                for (int v = w; v < nv; v += PS_WARPS)
+                {
+                    double c[3] = {0.0, 0.0, 0.0}; // coupled banks, isolated banks, coarse matrices
+#pragma unroll 1
+                    for (int j = v; j < ni; j += nv)
+                    {
+                        const Rec &it = rec[j];
+                        double d = 0.0;
+#pragma unroll
+                        for (int t = 0; t < BD; ++t)
+                            d = fma(it.yz[t * 32 + lane], it.r[t * 32 + lane], d);
+                        c[0] += it.m < mas.first_iso_bank ? d : 0.0;
+                        c[1] += it.m >= mas.first_iso_bank && it.m < banks ? d : 0.0;
+                        c[2] += it.m >= banks ? d : 0.0;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+                    {
+                        c[i] = warp_sum(c[i]);
+                        if (lane == 0)
+                            dot_rz[i * a.teams + v0 + v] = c[i];
+                    }
+                }
+                if (!(ok = ps_barrier(a.bar, target)))
+                    break;
+                // ---- Totals and the scalar step, in every CTA. The coarse corrections of the warp's first
+                // rows of p are on their way meanwhile.
+                double zc_next[4];
+                int4 slot_next = make_int4(-1, -1, -1, -1);
+                auto coarse_of = [&](int k) {
+                    const Rec &it = rec[k / BD];
+                    const int e = (k % BD) * 32 + lane, comp = e % BD;
+                    slot_next = it.cslot[e / BD];
+                    zc_next[0] = __ldcg(mas.zc + max(slot_next.x, 0) * BD + comp);
+                    zc_next[1] = __ldcg(mas.zc + max(slot_next.y, 0) * BD + comp);
+                    zc_next[2] = __ldcg(mas.zc + max(slot_next.z, 0) * BD + comp);
+                    zc_next[3] = __ldcg(mas.zc + max(slot_next.w, 0) * BD + comp);
+                };
+                if (w < nb * BD)
+                    coarse_of(w);
+                if (init)
+                {
+                    stage_dots(dot_bb, bank_pad, staged);
+                    __syncthreads();
+                    bank_dots_stage(staged, banks, sh.red + 8, w);
+                    __syncthreads();
+                }
+                stage_dots(dot_rr, a.staged, staged);
+                __syncthreads();
+                bank_dots_stage(staged, banks, sh.red, w);
+                for (int i = tid; i < 3 * a.vgrid; i += PS_THREADS)
+                {
+                    // Class i / vgrid of apply CTA c: its teams' dots in order.
+                    const int cls = i < a.vgrid ? 0 : (i < 2 * a.vgrid ? 1 : 2), c = i - cls * a.vgrid;
+                    const double *q = staged + bank_pad + cls * a.teams + c * L::TEAMS;
+                    double t = 0.0;
+#pragma unroll
+                    for (int k = 0; k < L::TEAMS; ++k)
+                        t += c * L::TEAMS + k < a.busy ? q[k] : 0.0;
+                    vpart[i] = t;
+                }
+                __syncthreads();
+                if (w < 3)
+                {
+                    // The last apply CTA's sum: TEAMS * 32 threads stride over the CTAs.
+                    const double *q = vpart + w * a.vgrid;
+                    double t = 0.0;
+#pragma unroll 1
+                    for (int k = 0; k < L::TEAMS && k * 32 < a.vgrid; ++k)
+                    {
+                        double s = 0.0;
+#pragma unroll 1
+                        for (int c = k * 32 + lane; c < a.vgrid; c += L::TEAMS * 32)
+                            s += q[c];
+                        t += warp_sum(s);
+                    }
+                    if (lane == 0)
+                        sh.tot[w] = t;
+                }
+                __syncthreads();
+                if (tid == 0)
+                {
+                    sh.st.rr = bank_total(sh.red);
+                    if (init)
+                        sh.st.rr0 = bank_total(sh.red + 8);
+                    const double Lc = (double)a.cfg.level_num;
+                    sh.st.rz_coarse = sh.tot[2] + Lc * sh.tot[1];
+                    sh.st.rzx_coarse = 0.0;
+                    pcg_finalize(&sh.st, a.cfg, init ? 1 : 2, sh.tot[0] + sh.tot[1] + sh.st.rz_coarse, 0.0);
+                }
+                __syncthreads();
+                // ---- x += alpha p (unless the true residual's update did it) and p = z + beta p.
+                const bool pdo = !__shfl_sync(FULL, sh.st.done, 0), xdo = !residual;
+                const double alpha = sh.st.alpha, beta = sh.st.beta;
+                const double iso_scale = 1.0 + mas.level_num;
+#pragma unroll 1
+                for (int k = w; k < nb * BD; k += PS_WARPS)
+                {
+                    Rec &it = rec[k / BD];
+                    const int e = (k % BD) * 32 + lane;
+                    const double po = it.p[e];
+                    if (xdo)
+                        it.x[e] = fma(alpha, po, it.x[e]);
+                    if (!pdo)
+                        continue;
+                    double v = it.yz[e];
+                    if (it.m < mas.first_iso_bank)
+                    {
+                        if (k != w)
+                            coarse_of(k);
+                        v += slot_next.x >= 0 ? zc_next[0] : 0.0;
+                        v += slot_next.y >= 0 ? zc_next[1] : 0.0;
+                        v += slot_next.z >= 0 ? zc_next[2] : 0.0;
+                        v += slot_next.w >= 0 ? zc_next[3] : 0.0;
+                    }
+                    else
+                        v = iso_scale * v;
+                    const double pn = init ? v : fma(beta, po, v);
+                    it.p[e] = pn;
+                    a.pg[(it.m * 32 + e / BD) * GATHER_STRIDE<BD> + e % BD] = pn;
+                }
+                if (!pdo || n + 1 == a.iters)
+                    break;
+                ok = ps_barrier(a.bar, target);
+            }
+
+            // ---- Out: x, r, the state; no copy may be in flight when the CTA leaves.
+            __syncthreads();
+#pragma unroll 1
+            for (int j = w; j < nb; j += PS_WARPS)
+#pragma unroll 1
+                for (int e = lane; e < N; e += 32)
+                {
+                    a.x[(size_t)rec[j].m * N + e] = rec[j].x[e];
+                    a.r[(size_t)rec[j].m * N + e] = rec[j].r[e];
+                }
+            if (tid == 0)
+            {
+#pragma unroll 1
+                for (long long i = 0; i < MBAR_SPIN_LIMIT; ++i)
+                    if (mbar_try_wait(&sh.bar, 0u))
+                        break;
+                if (!ok)
+                {
+                    sh.st.error = ERR_TIMEOUT;
+                    sh.st.done = 1;
+                }
+                if (blockIdx.x == 0)
+                    *a.st = sh.st;
+                else if (!ok)
+                    atomicExch(&a.st->error, ERR_TIMEOUT);
+            }
+        }
+
+        constexpr size_t PS_SMEM = 232448 - 1024; // dynamic shared memory beside the static part
+        static_assert(sizeof(PsShared) <= 1024, "static shared memory of the persistent solve");
+
+        template <int BD, class Store>
+        PersistPlan plan_variant(const MasView &mas)
+        {
+            using L = ApplyLayout<BD, Store>;
+            PersistPlan pl;
+            const int sms = device_sm_count();
+            const int items = mas.banks + mas.n_coarse_active;
+            // The dots are summed as the iteration kernels do for one bank per warp of update_xr.
+            if (mas.level_num < 1 || mas.banks < 1 || mas.banks > PERSIST_MAX_BANKS ||
+                update_xr_grid(mas) != (mas.banks + 7) / 8)
+                return pl;
+            pl.vgrid = mas_apply_grid(mas);
+            pl.teams = pl.vgrid * L::TEAMS;
+            pl.busy = pl.teams < items ? pl.teams : items;
+            pl.grid = pl.busy < sms ? pl.busy : sms;
+            pl.max_items = ((pl.busy + pl.grid - 1) / pl.grid) * ((items + pl.teams - 1) / pl.teams);
+            pl.deep_nodes = mas.real_count[1] + mas.real_count[2] + mas.real_count[3];
+            pl.staged = (((mas.banks + 7) & ~7) + 3 * pl.teams + 1) & ~1;
+            if (pl.deep_nodes < 0 || pl.deep_nodes > 1024 || mas.real_count[0] >= 0xFFFF)
+                return pl;
+            const size_t fixed = pl.max_items * (sizeof(ItemRec<BD>) + L::STAGE_BYTES) +
+                                 (size_t)PS_WARPS * PS_SCRATCH<BD, Store> +
+                                 (size_t)((3 * pl.vgrid + 1) & ~1) * sizeof(double) +
+                                 (size_t)((pl.deep_nodes * BD + 1) & ~1) * sizeof(double) +
+                                 (size_t)pl.staged * sizeof(double) + (size_t)pl.deep_nodes * 64;
+            if (fixed > PS_SMEM)
+                return pl;
+            pl.a_bytes = (int)((PS_SMEM - fixed) / 16 * 16);
+            pl.smem = fixed + pl.a_bytes;
+            pl.ok = true;
+            return pl;
+        }
+
+        template <class F>
+        auto dispatch_variant(int bd, int storage, F &&f)
+        {
+            switch (storage)
+            {
+            case STORE_F64:
+                return bd == 1 ? f.template operator()<1, double>()
+                               : (bd == 2 ? f.template operator()<2, double>() : f.template operator()<3, double>());
+            case STORE_F16:
+                return bd == 1 ? f.template operator()<1, __half>()
+                               : (bd == 2 ? f.template operator()<2, __half>() : f.template operator()<3, __half>());
+            default:
+                return bd == 1 ? f.template operator()<1, float>()
+                               : (bd == 2 ? f.template operator()<2, float>() : f.template operator()<3, float>());
+            }
+        }
+    } // namespace
+
+    // Every system whose inverses, vectors and coarse lists fit in the SMs' shared memory (290 banks of
+    // 96 x 96 FP64, 1,400 of FP16, 3,700 of 32 x 32): at each size measured up to there one launch was
+    // the faster path (the largest: 33^3 FP16 2,150 us against 3,060, 48^3 scalar FP16 3,930 against
+    // 4,250). Beyond, the inverses would stream from L2 through a ring: measured 1.2 to 2 times slower
+    // than the iteration kernels at 37^3 and 42^3.
+    PersistPlan persist_plan(const MasView &mas)
+    {
+        return dispatch_variant(mas.bd, mas.storage, [&]<int BD, class Store>() { return plan_variant<BD, Store>(mas); });
+    }
+
+    size_t persist_dots_size(const MasView &mas, const PersistPlan &pl)
+    {
+        return 2 * (size_t)((mas.banks + 7) & ~7) + (size_t)pl.staged;
+    }
+
+    size_t persist_gather_size(const MasView &mas)
+    {
+        return 2 * (size_t)mas.banks * 32 * (mas.bd == 3 ? 4 : mas.bd);
+    }
+
+    bool prepare_persistent(int bd, int storage)
+    {
+        return dispatch_variant(bd, storage, [&]<int BD, class Store>() {
+            int coop = 0, dev = 0, per_sm = 0;
+            cudaGetDevice(&dev);
+            if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+                cudaFuncSetAttribute(k_pcg_persistent<BD, Store>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)PS_SMEM) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_persistent<BD, Store>, PS_THREADS,
+                                                              PS_SMEM) != cudaSuccess ||
+                per_sm < 1)
+            {
+                cudaGetLastError();
+                return false;
+            }
+            return true;
+        });
+    }
+
+    void launch_pcg_persistent(const BankedView &A, const MasView &mas, const PcgConfig &cfg, const PersistPlan &pl,
+                               PcgState *st, double *x, double *r, double *gather, const double *b, double *dots,
+                               unsigned *bar, int first, int iters, int period, cudaStream_t s)
+    {
+        PersistArgs a{};
+        a.A = A;
+        a.mas = mas;
+        a.cfg = cfg;
+        a.st = st;
+        a.x = x;
+        a.r = r;
+        a.pg = gather;
+        a.xg = gather + persist_gather_size(mas) / 2;
+        a.b = b;
+        a.dots = dots;
+        a.bar = bar;
+        a.items = mas.banks + mas.n_coarse_active;
+        a.teams = pl.teams;
+        a.vgrid = pl.vgrid;
+        a.busy = pl.busy;
+        a.max_items = pl.max_items;
+        a.a_bytes = pl.a_bytes;
+        a.deep_nodes = pl.deep_nodes;
+        a.staged = pl.staged;
+        a.first = first;
+        a.iters = iters;
+        a.period = period;
+        cuda_check(cudaMemsetAsync(bar, 0, sizeof(unsigned), s), "barrier reset");
+        dispatch_variant(mas.bd, mas.storage, [&]<int BD, class Store>() {
+            void *args[] = {&a};
+            cuda_check(cudaLaunchCooperativeKernel((const void *)k_pcg_persistent<BD, Store>, dim3(pl.grid),
+                                                   dim3(PS_THREADS), args, pl.smem, s),
+                       "persistent solve launch");
+        });
+    }
+} // namespace pmas
