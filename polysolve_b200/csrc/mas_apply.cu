@@ -51,7 +51,7 @@ namespace pmas
             using Real = typename L::Real;
             constexpr int N = L::N, S = L::S, WARPS = L::WARPS;
             extern __shared__ __align__(128) unsigned char smem[];
-            const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const int w = warp_index(), lane = threadIdx.x & 31;
             unsigned char *base = smem + (size_t)w * L::TEAM_BYTES;
             Store *stage0 = reinterpret_cast<Store *>(base);
             Store *stage1 = reinterpret_cast<Store *>(base + L::STAGE_BYTES);
@@ -130,14 +130,7 @@ namespace pmas
                 double xscale = 1.0; // binary16 input: x * xscale split into hi + lo
                 if constexpr (L::MMA)
                 {
-                    double amax = 0.0;
-#pragma unroll
-                    for (int t = 0; t < BD; ++t)
-                        amax = fmax(amax, fabs(r64[t]));
-#pragma unroll
-                    for (int o = 16; o >= 1; o >>= 1)
-                        amax = fmax(amax, __shfl_xor_sync(FULL, amax, o));
-                    xscale = (amax > 0.0 && isfinite(amax)) ? ldexp(1.0, 14 - ilogb(amax)) : 1.0;
+                    xscale = half_scale<BD>(r64);
 #pragma unroll
                     for (int t = 0; t < BD; ++t)
                     {
@@ -180,7 +173,7 @@ namespace pmas
                 else
                     phase0 ^= 1u;
                 // Coarse matrices of isolated rows are exactly the identity: z = r, unrounded.
-                const bool ident = coarse && mas.identity[mat - banks];
+                const bool ident = coarse && warp_uniform(mas.identity[mat - banks]);
                 Real yr[BD];
                 if (!ident)
                 {
@@ -267,7 +260,7 @@ namespace pmas
             constexpr int N = L::N, S = L::S;
             extern __shared__ __align__(128) unsigned char smem[];
             __shared__ int team_failed[L::TEAMS];
-            const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const int w = warp_index(), lane = threadIdx.x & 31;
             const int team = w / BD, t = w - team * BD;
             unsigned char *base = smem + (size_t)team * L::TEAM_BYTES;
             double *xs = reinterpret_cast<double *>(base + 2 * L::STAGE_BYTES);
@@ -348,7 +341,7 @@ namespace pmas
                             zold[i] = out[i * 32 + lane];
                 }
                 // Coarse matrices of isolated rows are exactly the identity: z = r, unrounded.
-                const bool ident = coarse && mas.identity[mat - banks];
+                const bool ident = coarse && warp_uniform(mas.identity[mat - banks]);
                 if (!mbar_wait_bounded(&bar[s], s ? phase[1] : phase[0], errp, cfg.wait_limit) && lane == 0)
                     team_failed[team] = 1;
                 team_sync<BD>(team); // x complete; every warp has seen the copy or given up
@@ -560,7 +553,7 @@ namespace pmas
             if (grp->done)
                 return;
             extern __shared__ __align__(128) unsigned char smem[];
-            const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const int w = warp_index(), lane = threadIdx.x & 31;
             unsigned char *base = smem + (size_t)w * L::WARP_BYTES;
             __half *stage0 = reinterpret_cast<__half *>(base);
             __half *stage1 = reinterpret_cast<__half *>(base + L::STAGE_BYTES);
@@ -652,7 +645,7 @@ namespace pmas
                     phase1 ^= 1u;
                 else
                     phase0 ^= 1u;
-                const bool ident = coarse && mas.identity[mat - banks];
+                const bool ident = coarse && warp_uniform(mas.identity[mat - banks]);
                 if (!ident)
                     symv_mma16_g<BD>(stage, xh, xl, ys, lane);
                 __syncwarp();
@@ -756,7 +749,7 @@ namespace pmas
             if (grp->done)
                 return;
             extern __shared__ __align__(128) unsigned char smem[];
-            const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const int w = warp_index(), lane = threadIdx.x & 31;
             unsigned char *base = smem + (size_t)w * L::WARP_BYTES;
             __half *stage0 = reinterpret_cast<__half *>(base);
             __half *stage1 = reinterpret_cast<__half *>(base + L::STAGE_BYTES);
@@ -833,7 +826,7 @@ namespace pmas
                     phase1 ^= 1u;
                 else
                     phase0 ^= 1u;
-                const bool ident = coarse && mas.identity[mat - banks];
+                const bool ident = coarse && warp_uniform(mas.identity[mat - banks]);
                 if (!ident)
 #pragma unroll
                     for (int nt = 0; nt < G / 4; ++nt)
@@ -989,7 +982,7 @@ namespace pmas
             if (grp->done)
                 return;
             extern __shared__ __align__(1024) unsigned char smem[];
-            const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+            const int tid = threadIdx.x, w = warp_index(), lane = tid & 31;
             unsigned char *sA = smem, *sX = smem + L::OFF_X, *sB = smem + L::OFF_B;
             double *amax_s = reinterpret_cast<double *>(smem + L::OFF_AMAX);
             double *xsc_s = reinterpret_cast<double *>(smem + L::OFF_XSC);
@@ -1086,7 +1079,7 @@ namespace pmas
                     cat = mcat;
                 }
                 const double *x = reinterpret_cast<const double *>(sX + stg * L::X_BYTES);
-                const bool ident = coarse && mas.identity[mat - banks];
+                const bool ident = coarse && warp_uniform(mas.identity[mat - banks]);
                 double xv[12], am = 0.0;
 #pragma unroll
                 for (int i = 0; i < 12; ++i)
@@ -1262,7 +1255,7 @@ namespace pmas
             if (st && st->done)
                 return;
             constexpr int W = LEVEL_THREADS / 32;
-            const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const int w = warp_index(), lane = threadIdx.x & 31;
             __shared__ double part[W][BD];
             __shared__ int is_last;
             if (mas.level_num == 2)
@@ -1280,7 +1273,7 @@ namespace pmas
             }
             // Level-2 node j = cta.x; warp w: its w-th level-1 child.
             const int j = cta.x;
-            const int kb = mas.kid_ptr[2][j], ke = mas.kid_ptr[2][j + 1];
+            const int kb = warp_uniform(mas.kid_ptr[2][j]), ke = warp_uniform(mas.kid_ptr[2][j + 1]);
             if (kb + w < ke)
             {
                 const int i = mas.kids[kb + w];
@@ -1314,7 +1307,7 @@ namespace pmas
                 is_last = atomicAdd(mas.ticket, 1u) == (unsigned)cta.n - 1;
             }
             __syncthreads();
-            if (!is_last)
+            if (!warp_uniform(is_last))
                 return;
             __threadfence();
             for (int k = w; k < mas.real_count[3]; k += W)
@@ -1377,7 +1370,7 @@ namespace pmas
             if (grp && grp->done)
                 return;
             constexpr int W = LEVEL_THREADS / 32;
-            const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const int w = warp_index(), lane = threadIdx.x & 31;
             __shared__ double part[W][NC];
             __shared__ int is_last;
             if (mas.level_num == 2)
@@ -1397,7 +1390,7 @@ namespace pmas
                 return;
             }
             const int j = blockIdx.x;
-            const int kb = mas.kid_ptr[2][j], ke = mas.kid_ptr[2][j + 1];
+            const int kb = warp_uniform(mas.kid_ptr[2][j]), ke = warp_uniform(mas.kid_ptr[2][j + 1]);
             if (kb + w < ke)
             {
                 const int i = mas.kids[kb + w];
@@ -1431,7 +1424,7 @@ namespace pmas
                 is_last = atomicAdd(mas.ticket, 1u) == gridDim.x - 1;
             }
             __syncthreads();
-            if (!is_last)
+            if (!warp_uniform(is_last))
                 return;
             __threadfence();
             for (int k = w; k < mas.real_count[3]; k += W)
@@ -1461,7 +1454,7 @@ namespace pmas
             if (st && period > 0 && (st->iter + 1) % period != 0)
                 return;
             const int lane = threadIdx.x & 31;
-            const int bank = cta.x * 8 + (threadIdx.x >> 5);
+            const int bank = cta.x * 8 + warp_index();
             if (bank >= banks)
                 return;
             const long long b0 = (long long)bank * 32 * BD;

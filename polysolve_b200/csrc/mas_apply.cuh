@@ -272,6 +272,29 @@ namespace pmas
                 yr[t] = ys[t * 32 + lane];
         }
 
+        // The power of two that brings the warp's largest |v| to [2^14, 2^15) (1 for all zeros, or where it
+        // is not finite): the scale of the binary16 split. Only the exponent counts, so a 32-bit warp
+        // maximum of the high words finds it; denormal and non-finite maxima take the general way.
+        template <int BD>
+        __device__ __forceinline__ double half_scale(const double (&v)[BD])
+        {
+            unsigned hi = 0;
+#pragma unroll
+            for (int i = 0; i < BD; ++i)
+                hi = max(hi, (unsigned)__double2hiint(v[i]) & 0x7FFFFFFFu);
+            const unsigned e = __reduce_max_sync(FULL, hi) >> 20; // biased exponent
+            if (e >= 14 && e < 2047)
+                return __hiloint2double((int)((2060u - e) << 20), 0); // 2^(14 - (e - 1023))
+            double amax = 0.0;
+#pragma unroll
+            for (int i = 0; i < BD; ++i)
+                amax = fmax(amax, fabs(v[i]));
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1)
+                amax = fmax(amax, __shfl_xor_sync(FULL, amax, o));
+            return (amax > 0.0 && isfinite(amax)) ? ldexp(1.0, 14 - ilogb(amax)) : 1.0;
+        }
+
         // The reference's per-iteration scalar work and convergence test (MASSolver.cu:505,
         // 526-583), run by the last CTA of the apply. rz = r . z, rzcross = r . z_old (Polak-Ribiere).
         __device__ void pcg_finalize(PcgState *st, const PcgConfig &cfg, int mode, double rz, double rzcross)

@@ -104,7 +104,7 @@ namespace pmas
         __global__ void k_cco_lv0(BankedView A, const int *__restrict__ node_real, int *lcco0, int *cnt)
         {
             __shared__ unsigned sm[8][32];
-            const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+            const int lane = threadIdx.x & 31, w = warp_index();
             const int bank = blockIdx.x * 8 + w;
             if (bank >= A.banks)
                 return;
@@ -167,7 +167,7 @@ namespace pmas
         __global__ void k_cco_lvx(int C, const unsigned *__restrict__ masks, int *lid, int *cnt)
         {
             __shared__ unsigned sm[8][32];
-            const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+            const int lane = threadIdx.x & 31, w = warp_index();
             const int bank = blockIdx.x * 8 + w;
             const int c = bank * 32 + lane;
             if (bank * 32 >= C)
@@ -247,7 +247,7 @@ namespace pmas
             // step 3 touch disjoint elements (and the pivot records are free once step 2 is done).
             constexpr int KB = INV_KB;
             static_assert(N % KB == 0 && KB % 4 == 0, "pivot blocks of whole tiles");
-            const int lane = tid & 31, warp = tid >> 5;
+            const int lane = tid & 31, warp = warp_index();
             double *cd = coef;                // [KB] pivots
             double *cr = coef + KB;           // [KB][KB] pivot-row entries (0 at the pivot)
             double *cs = coef + KB + KB * KB; // [KB][KB] scaled entries

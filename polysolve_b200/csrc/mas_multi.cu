@@ -38,7 +38,7 @@ namespace pmas
             if (MODE == SPMV_RESIDUAL && period > 0 && (grp->iter + 1) % period != 0)
                 return;
             const int lane = threadIdx.x & 31;
-            const int bank = blockIdx.x * (MT / 32) + (threadIdx.x >> 5);
+            const int bank = blockIdx.x * (MT / 32) + warp_index();
             double part[G], bb[G];
 #pragma unroll
             for (int g = 0; g < G; ++g)
@@ -179,7 +179,7 @@ namespace pmas
 #pragma unroll
             for (int g = 0; g < G; ++g)
                 part[g] = 0.0;
-            for (int bank = blockIdx.x * (MT / 32) + (threadIdx.x >> 5); bank < mas.banks; bank += total_warps)
+            for (int bank = blockIdx.x * (MT / 32) + warp_index(); bank < mas.banks; bank += total_warps)
             {
                 const long long b0 = (long long)bank * 32 * BDG + lane;
                 double xv[BDG], pv[BDG], av[BDG], rv[BDG];
@@ -253,7 +253,7 @@ namespace pmas
             const int lane = threadIdx.x & 31;
             const double *__restrict__ zc = mas.zc;
             const double iso_scale = 1.0 + mas.level_num;
-            const int bank = blockIdx.x * (MT / 32) + (threadIdx.x >> 5);
+            const int bank = blockIdx.x * (MT / 32) + warp_index();
             if (bank >= mas.banks)
                 return;
             const long long b0 = (long long)bank * 32 * BDG;
@@ -328,7 +328,7 @@ namespace pmas
             if (period > 0 && (grp->iter + 1) % period != 0)
                 return;
             const int lane = threadIdx.x & 31;
-            const int bank = blockIdx.x * 8 + (threadIdx.x >> 5);
+            const int bank = blockIdx.x * 8 + warp_index();
             if (bank >= banks)
                 return;
             const long long b0 = (long long)bank * 32 * BDG;

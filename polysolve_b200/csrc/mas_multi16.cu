@@ -112,7 +112,7 @@ namespace pmas
                 return;
             if (MODE == SPMV_RESIDUAL && period > 0 && (grp->iter + 1) % period != 0)
                 return;
-            const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+            const int lane = threadIdx.x & 31, w = warp_index();
             const int rs = lane >> 3, gq = lane & 7; // row of the warp's four, pair of right-hand sides
             const int rb = w * 4 + rs;               // row within the bank
             const uint64_t pol = l2_evict_first_policy();
@@ -347,7 +347,7 @@ namespace pmas
             PcgState *grp = st + G;
             if (grp->done)
                 return;
-            const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+            const int lane = threadIdx.x & 31, w = warp_index();
             const double a = st[lane & (G - 1)].alpha;
             const bool due = period > 0 && (grp->iter + 1) % period == 0;
             if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -421,7 +421,7 @@ namespace pmas
                 return;
             if (period > 0 && (grp->iter + 1) % period != 0)
                 return;
-            const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+            const int lane = threadIdx.x & 31, w = warp_index();
             double *acc = xr_acc + (size_t)w * 32 * VN;
             for (int bank = blockIdx.x * WW + w; bank < mas.first_iso_bank; bank += gridDim.x * WW)
             {
@@ -454,7 +454,7 @@ namespace pmas
             if (grp->done && !xdo)
                 return;
             const int lane = threadIdx.x & 31;
-            const int bank = blockIdx.x * WW + (threadIdx.x >> 5);
+            const int bank = blockIdx.x * WW + warp_index();
             if (bank >= mas.banks)
                 return;
             const int g = lane & (G - 1);

@@ -52,7 +52,7 @@ namespace pmas
             constexpr int BS = BD * BD;
             constexpr int PAIRS = BS / 2;
             const int lane = threadIdx.x & 31;
-            const int bank = blockIdx.x * NOALLOC_BANKS_PER_CTA + (threadIdx.x >> 5);
+            const int bank = blockIdx.x * NOALLOC_BANKS_PER_CTA + warp_index();
             double part = 0.0;
             if (bank < A.banks)
             {

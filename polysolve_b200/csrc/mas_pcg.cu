@@ -132,7 +132,7 @@ namespace pmas
                     nbase = mas.cco0_base[bank];
                 }
             };
-            const int first = cta.x * (UPD_THREADS / 32) + (threadIdx.x >> 5);
+            const int first = cta.x * (UPD_THREADS / 32) + warp_index();
             if (first < mas.banks)
                 load(first);
             for (int bank = first; bank < mas.banks; bank += total_warps)
@@ -214,7 +214,7 @@ namespace pmas
             const int total_warps = cta.n * (UPD_THREADS / 32);
             const double *__restrict__ zc = mas.zc;
             const double iso_scale = 1.0 + mas.level_num;
-            for (int bank = cta.x * (UPD_THREADS / 32) + (threadIdx.x >> 5); bank < mas.banks; bank += total_warps)
+            for (int bank = cta.x * (UPD_THREADS / 32) + warp_index(); bank < mas.banks; bank += total_warps)
             {
                 const long long b0 = (long long)bank * 32 * BD;
                 if (bank >= mas.first_iso_bank)

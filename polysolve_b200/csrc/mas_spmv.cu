@@ -41,7 +41,7 @@ namespace pmas
             if (MODE == SPMV_RESIDUAL && period > 0 && (st->iter + 1) % period != 0)
                 return;
             const int lane = threadIdx.x & 31;
-            const int bank = cta.x * BANKS_PER_CTA + (threadIdx.x >> 5);
+            const int bank = cta.x * BANKS_PER_CTA + warp_index();
             double part = 0.0, bb = 0.0;
             if (bank < A.banks)
             {
@@ -234,7 +234,7 @@ namespace pmas
             constexpr int BS = BD * BD;
             constexpr int PAIRS = BS / 2;
             const int lane = threadIdx.x & 31;
-            const int bank = blockIdx.x * BANKS_PER_CTA + (threadIdx.x >> 5);
+            const int bank = blockIdx.x * BANKS_PER_CTA + warp_index();
             if (bank >= A.banks)
                 return;
             const int u = bank * 32 + lane;
