@@ -573,11 +573,12 @@ namespace pmas
     // once after a factorization; gather: persist_gather_size doubles (p and x as the SpMV gathers
     // them; kept between the launches of one solve); bar: one counter. first: start the solve, otherwise go on where the
     // launch before stopped; at most `iters` iterations per launch.
-    constexpr int PERSIST_MAX_BANKS = 4096;
+    constexpr int PERSIST_MAX_BANKS = 5200; // no plan beyond
     struct PersistPlan
     {
         bool ok = false;
-        int grid = 0, vgrid = 0, teams = 0, busy = 0, max_items = 0, a_bytes = 0, deep_nodes = 0, staged = 0;
+        int grid = 0, vgrid = 0, teams = 0, busy = 0, max_items = 0, slots = 0, ring = 0, batch = 0, a_bytes = 0, deep_nodes = 0,
+            staged = 0;
         size_t smem = 0;
     };
     bool prepare_persistent(int bd, int storage); // false: no cooperative launch of this shape here

@@ -1,10 +1,11 @@
 // The whole PCG solve of one system in one launch (sm_100a), for systems whose subdomain inverses fit
-// in the shared memory of all SMs. The iteration kernels of such a system are bound by latency:
-// launch, first loads and grid reduction, five times per iteration.
+// in the shared memory of all SMs, or nearly. The iteration kernels of such a system are bound by
+// latency: launch, first loads and grid reduction, five times per iteration.
 //
 // Every CTA (one per SM) owns a fixed set of work items for the whole solve: MAS subdomains (banks,
 // with their 32 block rows of the matrix and of x, r, p) and coarse matrices. It keeps in shared
-// memory the vectors of its rows, its inverses and as many of its matrix rows as fit. Only p
+// memory the vectors of its rows, its inverses (those that do not fit pass through a ring of bulk
+// copies, on their way while the CTA does something else) and as many of its matrix rows as fit. Only p
 // (gathered by the SpMV), the coarse vectors and the dot products pass through global memory, so an
 // iteration is four grid barriers:
 //
@@ -20,11 +21,11 @@
 // team m mod (grid * teams per CTA) -- for r.z). Each CTA computes all totals and the scalar step
 // itself.
 //
-// Measured (solve_device, us per solve, iteration kernels -> one launch): 20^3 elasticity FP16 1,870 ->
-// 955 (17 us per iteration), 33^3 FP16 3,060 -> 2,150, 200 x 100 plane FP16 3,850 -> 2,160, 30^3
-// scalar FP64 3,040 -> 1,720, 8^3 FP64 1,240 -> 640. An iteration at 20^3 is some 30,000 cycles: four
-// barriers of 2,400 (148 CTAs), 8,500 for the slowest CTA's SpMV (two rounds of gathers from L2), 4,000
-// for the totals and the scalar step, 7,000 for the coarse levels.
+// Measured: persist_plan below. An iteration at 20^3 is some 29,000 cycles: four barriers of 2,400 (148
+// CTAs), 3,500 for the SpMV (one round of gathers from L2), 4,500 for the totals and the scalar step,
+// 5,000 for the coarse levels.
+
+#include <algorithm>
 
 #include "mas_apply.cuh"
 
@@ -59,9 +60,11 @@ namespace pmas
             int vgrid;     // the apply's grid
             int busy;      // teams with work
             int max_items; // most items of a CTA
+            int slots, ring, batch; // shared-memory slots for inverses, how many of them are refilled, and how
+                                    // many at a time
             int a_bytes;   // shared memory for matrix rows (and the lists of the coarse sums)
             int deep_nodes; // nodes of the coarse levels above the first
-            int staged;     // dots staged at a time
+            int staged;     // shared memory of the staged dots (doubles)
             int first;      // start the solve (otherwise go on from st, x, r, p)
             int iters;      // iterations of this launch at most
             int period;     // true-residual period (0: never)
@@ -73,14 +76,15 @@ namespace pmas
         {
             double x[32 * BD], r[32 * BD], p[32 * BD];
             double yz[32 * BD]; // A p, then z
-            int4 cslot[32];
-            int key[32], len[32];
-            const double *avals; // matrix rows: values and columns (shared memory if resident)
+            ushort4 cslot[32]; // coarse nodes per level, 0xFFFF: none
+            int len[32];
+            signed char key[32];
+            const double *avals; // matrix rows: values and columns
             const int *acols;
             double scale;
             int m, mat;      // work item and matrix
             int ident;       // the inverse is exactly the identity
-            int resident;
+            int resident;    // 1 + offset of the rows' copy in shared memory, 0: none
             int width, base; // bank: slots per row, first component; coarse matrix above the first level:
                              // end of its level in `deep`, and the offset of a coarse node there
         };
@@ -89,8 +93,8 @@ namespace pmas
         {
             PcgState st;
             double red[16];
-            double tot[3];
-            uint64_t bar;
+            double tot[3][16]; // r.z by class, in parts
+            uint64_t bar, ring_bar[2];
             int deep_top, deep_lo, deep_hi; // coarse levels above the first: highest level this CTA needs,
                                             // its range of level-1 nodes
         };
@@ -140,11 +144,37 @@ namespace pmas
         }
 
         // Global dots (written before the last grid barrier) into shared memory, 16 bytes per thread and
-        // step: every CTA reads the same lines at the same time, so the number of requests counts.
-        __device__ __forceinline__ void stage_dots(const double *src, int count, double *dst)
+        // step: every CTA reads the same lines at the same time, so the number of requests counts. `eights`
+        // of them with one double of padding after every eight, `groups` with one after every GROUP (the
+        // threads that add a group each then hit different banks), the others as they are (GROUP 0: eights
+        // only). Counts even.
+        template <int GROUP>
+        __device__ __forceinline__ void stage_dots(const double *src, unsigned eights, unsigned groups, unsigned count,
+                                                   double *dst)
         {
-            for (int i = threadIdx.x * 2; i < count; i += PS_THREADS * 2)
-                *reinterpret_cast<double2 *>(dst + i) = __ldcg(reinterpret_cast<const double2 *>(src + i));
+            constexpr unsigned STEP = PS_THREADS * 2, U = 3;
+            const unsigned shift = eights / 8, tail = eights + groups, tail_shift = shift + groups / (GROUP ? GROUP : 1);
+            auto put = [&](unsigned i, double d) {
+                if constexpr (GROUP == 0)
+                    dst[i + i / 8] = d;
+                else
+                    dst[i + (i < eights ? i / 8 : (i < tail ? shift + (i - eights) / GROUP : tail_shift))] = d;
+            };
+#pragma unroll 1
+            for (unsigned i0 = threadIdx.x * 2; i0 < count; i0 += U * STEP)
+            {
+                double2 d[U];
+#pragma unroll
+                for (unsigned u = 0; u < U; ++u)
+                    d[u] = __ldcg(reinterpret_cast<const double2 *>(src + min(i0 + u * STEP, count - 2)));
+#pragma unroll
+                for (unsigned u = 0; u < U; ++u)
+                    if (i0 + u * STEP < count)
+                    {
+                        put(i0 + u * STEP, d[u].x);
+                        put(i0 + u * STEP + 1, d[u].y);
+                    }
+            }
         }
 
         // Sum of staged per-bank dots in the order of the SpMV's and update_xr's two-stage reduction (8
@@ -161,7 +191,7 @@ namespace pmas
                 double t = 0.0;
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    t += dots[g * 8 + i];
+                    t += dots[g * 9 + i];
                 s += t;
             }
             s = warp_sum(s);
@@ -208,7 +238,7 @@ namespace pmas
         // One bank's rows of y = A v by one warp (lane = block row). v was written by other CTAs before
         // the last grid barrier. RES: the rows are in shared memory, so only the gathers of v take
         // time: U of them in flight. Otherwise everything comes from L2. Slots past a row's end hold
-        // column 0; their products are not added.
+        // column 0 and zero values, which add zero.
         template <int BD, int U, bool RES>
         __device__ __forceinline__ void bank_rows(const double *vp, const int *cp, int len, int width, const double *v,
                                                   int lane, double (&acc)[BD])
@@ -247,6 +277,11 @@ namespace pmas
 #pragma unroll
                 for (int u = 0; u < U; ++u)
                     cn[u] = k0 + U + u < width ? (RES ? cp[(k0 + U + u) * 32] : __ldg(cp + (k0 + U + u) * 32)) : 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int j = 0; j < BD; ++j)
+                        xc[u][j] = k0 + u < len ? xc[u][j] : 0.0;
                 if (RES)
                     load_block(k0, m[0]);
 #pragma unroll
@@ -254,15 +289,11 @@ namespace pmas
                 {
                     if (RES && u + 1 < U)
                         load_block(min(k0 + u + 1, width - 1), m[RES ? (u + 1) & 1 : 0]);
-                    const bool in = k0 + u < len;
 #pragma unroll
                     for (int i = 0; i < BD; ++i)
 #pragma unroll
                         for (int j = 0; j < BD; ++j)
-                        {
-                            const double t = fma(m[RES ? u & 1 : u][i * BD + j], xc[u][j], acc[i]);
-                            acc[i] = in ? t : acc[i];
-                        }
+                            acc[i] = fma(m[RES ? u & 1 : u][i * BD + j], xc[u][j], acc[i]);
                 }
             }
         }
@@ -320,38 +351,102 @@ namespace pmas
             return ys[lane];
         }
 
+        // Rows 32 t .. 32 t + 31 of z = M r for one work item by one warp. The item's record, its inverse M and
+        // the warp's scratch are given as offsets in shared memory (as pointers they would be read through
+        // generic addresses in a function of its own).
+        template <int BD, class Store>
+        __device__ __noinline__ void apply_rows(unsigned rec_at, unsigned inv_at, unsigned scratch_at, int t, int lane,
+                                                int banks, double *zc)
+        {
+            using L = ApplyLayout<BD, Store>;
+            using Real = typename L::Real;
+            constexpr int N = L::N;
+            extern __shared__ __align__(128) unsigned char smem[];
+            ItemRec<BD> &it = *reinterpret_cast<ItemRec<BD> *>(smem + rec_at);
+            const Store *M = reinterpret_cast<const Store *>(smem + inv_at);
+            unsigned char *scratch = smem + scratch_at;
+            const int e = t * 32 + lane;
+            double zv;
+            if constexpr (L::MMA)
+            {
+                __half *xh = reinterpret_cast<__half *>(scratch), *xl = xh + N;
+                double rv[BD];
+#pragma unroll
+                for (int i = 0; i < BD; ++i)
+                    rv[i] = it.r[i * 32 + lane];
+                const double xscale = half_scale<BD>(rv);
+#pragma unroll
+                for (int i = 0; i < BD; ++i)
+                {
+                    const float f = (float)(rv[i] * xscale);
+                    const __half h = __float2half_rn(f);
+                    xh[i * 32 + lane] = h;
+                    xl[i * 32 + lane] = __float2half_rn(f - __half2float(h));
+                }
+                __syncwarp();
+                zv = (double)symv_mma16_rows<BD>(M, xh, xl, reinterpret_cast<float *>(xl + N), t, lane) *
+                     (it.scale / xscale);
+            }
+            else if constexpr (std::is_same_v<Real, double>)
+                zv = symv_row<BD>(M, it.r, t, lane);
+            else
+            {
+                float *xs = reinterpret_cast<float *>(scratch);
+#pragma unroll
+                for (int i = 0; i < BD; ++i)
+                    xs[i * 32 + lane] = (float)it.r[i * 32 + lane];
+                __syncwarp();
+                zv = (double)symv_row<BD>(M, xs, t, lane);
+            }
+            if (it.ident)
+                zv = it.r[e];
+            it.yz[e] = zv;
+            if (it.m >= banks)
+                zc[(size_t)(it.mat - banks) * N + e] = zv;
+            __syncwarp(); // the scratch is read
+        }
+
         template <int BD, class Store>
         __global__ void __launch_bounds__(PS_THREADS, 1) k_pcg_persistent(const __grid_constant__ PersistArgs a)
         {
             using L = ApplyLayout<BD, Store>;
-            using Real = typename L::Real;
             using Rec = ItemRec<BD>;
             constexpr int N = L::N, BS = BD * BD;
             extern __shared__ __align__(128) unsigned char smem[];
             __shared__ PsShared sh;
-            // The warp index as a broadcast, so that the compiler knows it to be uniform in the warp: in
-            // branches and loops that it cannot prove uniform it guards every shuffle, and a warp sum
-            // takes 2,500 cycles instead of 250.
-            const int tid = threadIdx.x, w = __shfl_sync(FULL, tid >> 5, 0), lane = tid & 31;
+            const int tid = threadIdx.x, w = warp_index(), lane = tid & 31;
             const MasView &mas = a.mas;
             const int banks = mas.banks;
 
-            // ---- The CTA's items: teams [v0, v0 + nv), item j = (k, v) in increasing order (item m =
-            // v0 + v + k * teams), so its nb banks come before its coarse matrices.
-            const int v0 = (int)((long long)blockIdx.x * a.busy / gridDim.x);
-            const int nv = (int)((long long)(blockIdx.x + 1) * a.busy / gridDim.x) - v0;
-            int ni = 0, nb = 0;
-#pragma unroll 1
-            for (int k = v0; k < a.items; k += a.teams)
+            // ---- The CTA's items, banks first. With a team per item (single): a contiguous share of the banks
+            // (neighbours gather from one another) and every gridDim.x-th coarse matrix, from the last CTA
+            // down. Otherwise every gridDim.x-th team from the CTA's index on, item j = (k, i) in increasing
+            // order (item m = blockIdx.x + i * gridDim.x + k * teams).
+            const int G = (int)gridDim.x, back = G - 1 - (int)blockIdx.x;
+            const bool single = a.busy == a.items;
+            const int b0 = single ? (int)((long long)blockIdx.x * banks / G) : (int)blockIdx.x;
+            int nb, ni, nv; // banks, items, teams
+            if (single)
             {
-                ni += min(nv, a.items - k);
-                nb += max(0, min(nv, banks - k));
+                nb = (int)((long long)(blockIdx.x + 1) * banks / G) - b0;
+                nv = ni = nb + (a.items - banks - back + G - 1) / G;
+            }
+            else
+            {
+                nv = (a.busy - b0 + G - 1) / G;
+                nb = ni = 0;
+#pragma unroll 1
+                for (int k = b0; k < a.items; k += a.teams)
+                {
+                    ni += min(nv, (a.items - k + G - 1) / G);
+                    nb += max(0, min(nv, (banks - k + G - 1) / G));
+                }
             }
 
             // ---- Shared memory.
             Rec *rec = reinterpret_cast<Rec *>(smem);
             unsigned char *at = smem + (size_t)a.max_items * sizeof(Rec);
-            unsigned char *scratch = at + (size_t)w * PS_SCRATCH<BD, Store>;
+            const unsigned scratch_at = (unsigned)(at - smem) + (unsigned)w * PS_SCRATCH<BD, Store>;
             at += (size_t)PS_WARPS * PS_SCRATCH<BD, Store>;
             double *vpart = reinterpret_cast<double *>(at); // 3 * vgrid partials of the apply's dots
             at += (size_t)((3 * a.vgrid + 1) & ~1) * sizeof(double);
@@ -362,11 +457,30 @@ namespace pmas
             unsigned short *kids = reinterpret_cast<unsigned short *>(at); // children of the nodes of `deep`
             at += (size_t)a.deep_nodes * 64;
             unsigned char *slots = at; // the inverses
-            unsigned char *a_rows = slots + (size_t)a.max_items * L::STAGE_BYTES;
+            unsigned char *a_rows = slots + (size_t)a.slots * L::STAGE_BYTES;
             const unsigned char *inv = static_cast<const unsigned char *>(mas.inv);
+            // Inverse slots: the coarse matrices and the first `kept` banks keep theirs. Where the other
+            // banks' do not fit, they pass through the last slots in batches (at most one round of the
+            // CTA's warps), batch g (counted over the launch) through buffer g mod `buffers`.
+            const int per = a.batch;
+            const int buffers = ni <= a.slots ? 0 : a.ring / per;
+            const int kept = buffers ? a.slots - a.ring - (ni - nb) : nb;
+            const int batches = (nb - kept + per - 1) / per;
+            unsigned char *ring = slots + (size_t)(a.slots - a.ring) * L::STAGE_BYTES;
+            // Slot of a kept item: coarse ones first.
+            auto slot_of = [&](int j) { return slots + (size_t)(j < nb ? ni - nb + j : j - nb) * L::STAGE_BYTES; };
+            auto load_batch = [&](int g) {
+                const int first = kept + g % batches * per, n = min(per, nb - first);
+                uint64_t *bar = &sh.ring_bar[g % buffers];
+                mbar_arrive_expect_tx(bar, (uint32_t)(n * L::STAGE_BYTES));
+                for (int i = 0; i < n; ++i)
+                    bulk_copy_g2s(ring + (size_t)(g % buffers * per + i) * L::STAGE_BYTES,
+                                  inv + (size_t)rec[first + i].mat * L::STAGE_BYTES, L::STAGE_BYTES, bar);
+            };
 
             double *dot_pap = a.dots;
-            const int bank_pad = (banks + 7) & ~7;
+            const int bank_pad = (banks + 7) & ~7, team_pad = (a.busy + 1) & ~1;
+            const int extras = a.items - mas.first_iso_bank, first_extra = mas.first_iso_bank % a.teams;
             double *dot_bb = a.dots + bank_pad, *dot_rr = a.dots + 2 * bank_pad, *dot_rz = a.dots + 3 * bank_pad;
 
             // ---- Load the CTA's part of the system.
@@ -374,6 +488,8 @@ namespace pmas
             {
                 sh.deep_top = sh.deep_lo = sh.deep_hi = 0;
                 mbar_init(&sh.bar, 1);
+                mbar_init(&sh.ring_bar[0], 1);
+                mbar_init(&sh.ring_bar[1], 1);
                 fence_mbar_init();
                 unsigned *z = reinterpret_cast<unsigned *>(&sh.st);
                 const unsigned *src = reinterpret_cast<const unsigned *>(a.st);
@@ -385,7 +501,7 @@ namespace pmas
             for (int j = w; j < ni; j += PS_WARPS)
             {
                 Rec &it = rec[j];
-                const int m = v0 + j % nv + (j / nv) * a.teams;
+                const int m = single ? (j < nb ? b0 + j : banks + back + (j - nb) * G) : b0 + j % nv * G + j / nv * a.teams;
                 if (lane == 0)
                 {
                     it.m = m;
@@ -396,8 +512,10 @@ namespace pmas
                 if (m >= banks)
                     continue;
                 it.len[lane] = a.A.rowlen[m * 32 + lane];
-                it.key[lane] = m < mas.first_iso_bank ? mas.lcco0[m * 32 + lane] : -1;
-                it.cslot[lane] = mas.cslot[m * 32 + lane];
+                it.key[lane] = m < mas.first_iso_bank ? (signed char)mas.lcco0[m * 32 + lane] : -1;
+                const int4 cs = mas.cslot[m * 32 + lane];
+                it.cslot[lane] = make_ushort4((unsigned short)cs.x, (unsigned short)cs.y, (unsigned short)cs.z,
+                                              (unsigned short)cs.w);
 #pragma unroll 1
                 for (int e = lane; e < N; e += 32)
                 {
@@ -429,25 +547,25 @@ namespace pmas
                     const int bytes = rec[j].width * 32 * (BS * 8 + 4);
                     if (bytes > 0 && used + bytes <= a.a_bytes)
                     {
-                        rec[j].resident = 1;
+                        rec[j].resident = 1 + used;
                         used += bytes;
                     }
                 }
-                mbar_arrive_expect_tx(&sh.bar, (uint32_t)(used + ni * L::STAGE_BYTES));
-                used = 0;
+                mbar_arrive_expect_tx(&sh.bar, (uint32_t)(used + (kept + ni - nb) * L::STAGE_BYTES));
+#pragma unroll 1
+                for (int g = 0; g < buffers; ++g)
+                    load_batch(g);
 #pragma unroll 1
                 for (int j = 0; j < ni; ++j)
                 {
-                    bulk_copy_g2s(slots + (size_t)j * L::STAGE_BYTES, inv + (size_t)rec[j].mat * L::STAGE_BYTES,
-                                  L::STAGE_BYTES, &sh.bar);
+                    if (j < kept || j >= nb)
+                        bulk_copy_g2s(slot_of(j), inv + (size_t)rec[j].mat * L::STAGE_BYTES, L::STAGE_BYTES, &sh.bar);
                     if (j >= nb || !rec[j].resident)
                         continue;
                     const uint32_t vb = (uint32_t)rec[j].width * 32 * BS * 8, cb = (uint32_t)rec[j].width * 32 * 4;
-                    bulk_copy_g2s(a_rows + used, rec[j].avals, vb, &sh.bar);
-                    bulk_copy_g2s(a_rows + used + vb, rec[j].acols, cb, &sh.bar);
-                    rec[j].avals = reinterpret_cast<const double *>(a_rows + used);
-                    rec[j].acols = reinterpret_cast<const int *>(a_rows + used + vb);
-                    used += vb + cb;
+                    unsigned char *to = a_rows + rec[j].resident - 1;
+                    bulk_copy_g2s(to, rec[j].avals, vb, &sh.bar);
+                    bulk_copy_g2s(to + vb, rec[j].acols, cb, &sh.bar);
                 }
                 // The coarse sums above the first level that this CTA's coarse matrices take.
 #pragma unroll 1
@@ -479,8 +597,10 @@ namespace pmas
             if (!ok && tid == 0)
                 atomicOr(a.bar, PS_ABORT);
             unsigned target = 0;
-            const int deep_top = __shfl_sync(FULL, sh.deep_top, 0), deep_lo = __shfl_sync(FULL, sh.deep_lo, 0),
-                      deep_hi = __shfl_sync(FULL, sh.deep_hi, 0);
+            int batch = 0; // batches multiplied in this launch
+            bool gave_up = false; // a wait for a batch ran out
+            const int deep_top = warp_uniform(sh.deep_top), deep_lo = warp_uniform(sh.deep_lo),
+                      deep_hi = warp_uniform(sh.deep_hi);
             {
                 int to = 0; // the level's first node
 #pragma unroll 1
@@ -515,10 +635,14 @@ namespace pmas
 #pragma unroll
                         for (int i = 0; i < BD; ++i)
                             acc[i] = 0.0;
-                        if (__shfl_sync(FULL, it.resident, 0))
-                            bank_rows<BD, 8, true>(it.avals, it.acols, it.len[lane], __shfl_sync(FULL, it.width, 0), v, lane, acc);
+                        const int width = warp_uniform(it.width), copy = warp_uniform(it.resident);
+                        if (copy)
+                            bank_rows<BD, BD == 3 ? 15 : 9, true>(
+                                reinterpret_cast<const double *>(a_rows + copy - 1),
+                                reinterpret_cast<const int *>(a_rows + copy - 1 + width * 32 * BS * 8), it.len[lane], width, v,
+                                lane, acc);
                         else
-                            bank_rows<BD, BD == 3 ? 3 : 4, false>(it.avals, it.acols, it.len[lane], __shfl_sync(FULL, it.width, 0), v, lane, acc);
+                            bank_rows<BD, BD == 3 ? 5 : 8, false>(it.avals, it.acols, it.len[lane], width, v, lane, acc);
 #pragma unroll
                         for (int i = 0; i < BD; ++i)
                         {
@@ -548,13 +672,13 @@ namespace pmas
                         break;
                     if (!(ok = ps_barrier(a.bar, target)))
                         break;
-                    stage_dots(dot_pap, bank_pad, staged);
+                    stage_dots<0>(dot_pap, bank_pad, 0, bank_pad, staged);
                     __syncthreads();
                     bank_dots_stage(staged, banks, sh.red, w);
                     __syncthreads();
                     const double pap = bank_total(sh.red);
                     const double alpha = (fabs(pap) < 1e-20) ? 0.0 : sh.st.rz / pap;
-                    residual = a.period > 0 && (__shfl_sync(FULL, sh.st.iter, 0) + 1) % a.period == 0;
+                    residual = a.period > 0 && (warp_uniform(sh.st.iter) + 1) % a.period == 0;
                     if (tid == 0)
                     {
                         sh.st.pAp = pap;
@@ -601,7 +725,7 @@ namespace pmas
                 for (int j = w; j < nb; j += PS_WARPS)
                 {
                     Rec &it = rec[j];
-                    if (__shfl_sync(FULL, it.m, 0) >= mas.first_iso_bank)
+                    if (warp_uniform(it.m) >= mas.first_iso_bank)
                         continue;
                     double rv[BD];
 #pragma unroll
@@ -620,39 +744,41 @@ namespace pmas
                     {
                         if (!(ok = ps_wait(a.bar, target)) || nb == ni)
                             break;
-                        // Coarse levels above the first: a warp per node, lane = child (the order of
-                        // k_coarse_levels), two nodes at a time.
+                        // Coarse levels above the first, four nodes per warp: eight lanes per node, four of its
+                        // children each, added in the order of the warp sums of k_coarse_levels (children 16
+                        // apart first, then 8, 4, 2, 1; absent ones are zero).
                         int from = 0, to = 0; // first node of the level below and of the level
 #pragma unroll 1
                         for (int l = 1; l <= deep_top; ++l)
                         {
                             const int hi = l == 1 ? deep_hi : mas.real_count[l];
 #pragma unroll 1
-                            for (int i = (l == 1 ? deep_lo : 0) + w; i < hi; i += 2 * PS_WARPS)
+                            for (int i = (l == 1 ? deep_lo : 0) + w * 4; i < hi; i += PS_WARPS * 4)
                             {
-                                double t[2][BD];
+                                const int node = i + (lane >> 3), s8 = lane & 7;
+                                double t[4][BD];
 #pragma unroll
-                                for (int h = 0; h < 2; ++h)
+                                for (int h = 0; h < 4; ++h)
                                 {
-                                    const int kid = i + h * PS_WARPS < hi ? kids[(to + i + h * PS_WARPS) * 32 + lane] : 0xFFFF;
+                                    const int q = node < hi ? kids[(to + node) * 32 + s8 + 8 * h] : 0xFFFF;
+                                    const int at = (q == 0xFFFF ? 0 : (l == 1 ? mas.coff[0] : from) + q) * BD;
 #pragma unroll
                                     for (int c = 0; c < BD; ++c)
                                     {
-                                        t[h][c] = 0.0;
-                                        if (kid != 0xFFFF)
-                                            t[h][c] = l == 1 ? __ldcg(mas.rc + (mas.coff[0] + kid) * BD + c)
-                                                             : deep[(from + kid) * BD + c];
+                                        const double v = l == 1 ? __ldcg(mas.rc + at + c) : deep[at + c];
+                                        t[h][c] = q == 0xFFFF ? 0.0 : v;
                                     }
                                 }
 #pragma unroll
-                                for (int h = 0; h < 2; ++h)
+                                for (int c = 0; c < BD; ++c)
+                                {
+                                    double v = (t[0][c] + t[2][c]) + (t[1][c] + t[3][c]);
 #pragma unroll
-                                    for (int c = 0; c < BD; ++c)
-                                    {
-                                        t[h][c] = warp_sum(t[h][c]);
-                                        if (lane == 0 && i + h * PS_WARPS < hi)
-                                            deep[(to + i + h * PS_WARPS) * BD + c] = t[h][c];
-                                    }
+                                    for (int o = 4; o >= 1; o >>= 1)
+                                        v += __shfl_xor_sync(FULL, v, o);
+                                    if (s8 == 0 && node < hi)
+                                        deep[(to + node) * BD + c] = v;
+                                }
                             }
                             __syncthreads();
                             from = to;
@@ -669,67 +795,46 @@ namespace pmas
                         }
                         __syncthreads();
                     }
-                    const int j0 = part ? nb : 0, tasks = (part ? ni - nb : nb) * BD;
+                    // 32 rows of one matrix per warp: the kept ones, then (part 0) batch by batch.
+                    const int j0 = part ? nb : 0, tasks = (part ? ni - nb : kept) * BD;
 #pragma unroll 1
                     for (int k = w; k < tasks; k += PS_WARPS)
+                        apply_rows<BD, Store>((j0 + k / BD) * (unsigned)sizeof(Rec), (unsigned)(slot_of(j0 + k / BD) - smem), scratch_at,
+                                              k % BD, lane, banks, mas.zc);
+                    const int end = part || buffers == 0 ? 0 : batches;
+#pragma unroll 1
+                    for (int done = 0; done < end; ++done, ++batch)
                     {
-                        const int j = j0 + k / BD, t = k % BD, e = t * 32 + lane;
-                        Rec &it = rec[j];
-                        const Store *M = reinterpret_cast<const Store *>(slots + (size_t)j * L::STAGE_BYTES);
-                        double zv;
-                        if constexpr (L::MMA)
+                        const int j = kept + done * per + w / BD;
+                        if (!mbar_wait_bounded(&sh.ring_bar[batch % buffers], (uint32_t)(batch / buffers) & 1u, nullptr,
+                                               a.cfg.wait_limit))
+                            gave_up = true;
+                        if (w / BD < per && j < nb)
+                            apply_rows<BD, Store>(
+                                j * (unsigned)sizeof(Rec),
+                                (unsigned)(ring - smem) + (unsigned)(batch % buffers * per + w / BD) * L::STAGE_BYTES,
+                                scratch_at, w % BD, lane, banks, mas.zc);
+                        // Every warp is done with the batch: its buffer takes the batch `buffers` on.
+                        if (__syncthreads_or(gave_up))
+                            break;
+                        if (tid == 0)
                         {
-                            __half *xh = reinterpret_cast<__half *>(scratch), *xl = xh + N;
-                            double rv[BD], amax = 0.0;
-#pragma unroll
-                            for (int i = 0; i < BD; ++i)
-                            {
-                                rv[i] = it.r[i * 32 + lane];
-                                amax = fmax(amax, fabs(rv[i]));
-                            }
-#pragma unroll
-                            for (int o = 16; o >= 1; o >>= 1)
-                                amax = fmax(amax, __shfl_xor_sync(FULL, amax, o));
-                            const double xscale = (amax > 0.0 && isfinite(amax)) ? ldexp(1.0, 14 - ilogb(amax)) : 1.0;
-#pragma unroll
-                            for (int i = 0; i < BD; ++i)
-                            {
-                                const float f = (float)(rv[i] * xscale);
-                                const __half h = __float2half_rn(f);
-                                xh[i * 32 + lane] = h;
-                                xl[i * 32 + lane] = __float2half_rn(f - __half2float(h));
-                            }
-                            __syncwarp();
-                            zv = (double)symv_mma16_rows<BD>(M, xh, xl, reinterpret_cast<float *>(xl + N), t, lane) *
-                                 (it.scale / xscale);
+                            fence_proxy_async_smem();
+                            load_batch(batch + buffers);
                         }
-                        else if constexpr (std::is_same_v<Real, double>)
-                            zv = symv_row<BD>(M, it.r, t, lane);
-                        else
-                        {
-                            float *xs = reinterpret_cast<float *>(scratch);
-#pragma unroll
-                            for (int i = 0; i < BD; ++i)
-                                xs[i * 32 + lane] = (float)it.r[i * 32 + lane];
-                            __syncwarp();
-                            zv = (double)symv_row<BD>(M, xs, t, lane);
-                        }
-                        if (it.ident)
-                            zv = it.r[e];
-                        it.yz[e] = zv;
-                        if (part == 1)
-                            mas.zc[(size_t)(it.mat - banks) * N + e] = zv;
-                        __syncwarp(); // the scratch is read
                     }
                 }
                 if (!ok)
                     break;
-                __syncthreads();
-                // ---- r.z per team: its items in order, then the warp sum.
+                if (__syncthreads_or(gave_up) && tid == 0)
+                    atomicOr(a.bar, PS_ABORT); // barrier C below tells every CTA
+                // ---- r.z per team: its coupled banks in order, then the warp sum. A team has at most one item
+                // beyond them (an isolated bank or a coarse matrix): its dot on its own, by item.
 #pragma unroll 1
                 for (int v = w; v < nv; v += PS_WARPS)
                 {
-                    double c[3] = {0.0, 0.0, 0.0}; // coupled banks, isolated banks, coarse matrices
+                    double c = 0.0, beyond = 0.0;
+                    int extra = -1;
 #pragma unroll 1
                     for (int j = v; j < ni; j += nv)
                     {
@@ -738,16 +843,22 @@ namespace pmas
 #pragma unroll
                         for (int t = 0; t < BD; ++t)
                             d = fma(it.yz[t * 32 + lane], it.r[t * 32 + lane], d);
-                        c[0] += it.m < mas.first_iso_bank ? d : 0.0;
-                        c[1] += it.m >= mas.first_iso_bank && it.m < banks ? d : 0.0;
-                        c[2] += it.m >= banks ? d : 0.0;
+                        const int m = warp_uniform(it.m);
+                        if (m < mas.first_iso_bank)
+                            c += d;
+                        else
+                        {
+                            beyond = d;
+                            extra = m - mas.first_iso_bank;
+                        }
                     }
-#pragma unroll
-                    for (int i = 0; i < 3; ++i)
+                    c = warp_sum(c);
+                    beyond = warp_sum(beyond);
+                    if (lane == 0)
                     {
-                        c[i] = warp_sum(c[i]);
-                        if (lane == 0)
-                            dot_rz[i * a.teams + v0 + v] = c[i];
+                        dot_rz[rec[v].m] = c;
+                        if (extra >= 0)
+                            dot_rz[team_pad + extra] = beyond;
                     }
                 }
                 if (!(ok = ps_barrier(a.bar, target)))
@@ -755,56 +866,75 @@ namespace pmas
                 // ---- Totals and the scalar step, in every CTA. The coarse corrections of the warp's first
                 // rows of p are on their way meanwhile.
                 double zc_next[4];
-                int4 slot_next = make_int4(-1, -1, -1, -1);
+                ushort4 slot_next;
                 auto coarse_of = [&](int k) {
                     const Rec &it = rec[k / BD];
-                    const int e = (k % BD) * 32 + lane, comp = e % BD;
+                    const int e = (k % BD) * 32 + lane;
+                    const double *zc = mas.zc + e % BD;
                     slot_next = it.cslot[e / BD];
-                    zc_next[0] = __ldcg(mas.zc + max(slot_next.x, 0) * BD + comp);
-                    zc_next[1] = __ldcg(mas.zc + max(slot_next.y, 0) * BD + comp);
-                    zc_next[2] = __ldcg(mas.zc + max(slot_next.z, 0) * BD + comp);
-                    zc_next[3] = __ldcg(mas.zc + max(slot_next.w, 0) * BD + comp);
+                    auto value = [&](unsigned short q) { return __ldcg(zc + (q == 0xFFFF ? 0 : q) * BD); };
+                    zc_next[0] = value(slot_next.x);
+                    zc_next[1] = value(slot_next.y);
+                    zc_next[2] = value(slot_next.z);
+                    zc_next[3] = value(slot_next.w);
                 };
                 if (w < nb * BD)
                     coarse_of(w);
                 if (init)
                 {
-                    stage_dots(dot_bb, bank_pad, staged);
+                    stage_dots<0>(dot_bb, bank_pad, 0, bank_pad, staged);
                     __syncthreads();
                     bank_dots_stage(staged, banks, sh.red + 8, w);
                     __syncthreads();
                 }
-                stage_dots(dot_rr, a.staged, staged);
+                double *staged_rz = staged + bank_pad / 8 * 9;
+                stage_dots<L::TEAMS>(dot_rr, bank_pad, team_pad, bank_pad + team_pad + ((extras + 1) & ~1), staged);
                 __syncthreads();
                 bank_dots_stage(staged, banks, sh.red, w);
                 for (int i = tid; i < 3 * a.vgrid; i += PS_THREADS)
                 {
                     // Class i / vgrid of apply CTA c: its teams' dots in order.
                     const int cls = i < a.vgrid ? 0 : (i < 2 * a.vgrid ? 1 : 2), c = i - cls * a.vgrid;
-                    const double *q = staged + bank_pad + cls * a.teams + c * L::TEAMS;
                     double t = 0.0;
+                    if (cls == 0)
+                    {
+                        const double *q = staged_rz + c * (L::TEAMS + 1);
 #pragma unroll
-                    for (int k = 0; k < L::TEAMS; ++k)
-                        t += c * L::TEAMS + k < a.busy ? q[k] : 0.0;
+                        for (int k = 0; k < L::TEAMS; ++k)
+                            t += c * L::TEAMS + k < a.busy ? q[k] : 0.0;
+                    }
+                    else
+                    {
+                        // The items beyond the coupled banks: team first_iso_bank mod teams has the first.
+                        const double *q = staged_rz + team_pad + team_pad / L::TEAMS;
+                        const int lo = cls == 1 ? 0 : banks - mas.first_iso_bank;
+                        const int hi = cls == 1 ? banks - mas.first_iso_bank : extras;
+                        const int x0 = c * L::TEAMS - first_extra;
+                        if ((x0 + L::TEAMS > lo && x0 < hi) || (x0 < 0 && x0 + a.teams < hi))
+#pragma unroll
+                            for (int k = 0; k < L::TEAMS; ++k)
+                            {
+                                const int x = x0 + k < 0 ? x0 + k + a.teams : x0 + k;
+                                t += x >= lo && x < hi ? q[x] : 0.0;
+                            }
+                    }
                     vpart[i] = t;
                 }
                 __syncthreads();
-                if (w < 3)
+                // The last apply CTA's sum: TEAMS * 32 threads stride over the CTAs, a warp sum each 32,
+                // added in order (by thread 0 below).
+                const int rounds = min(L::TEAMS, (a.vgrid + 31) / 32);
+#pragma unroll 1
+                for (int k = w; k < 3 * rounds; k += PS_WARPS)
                 {
-                    // The last apply CTA's sum: TEAMS * 32 threads stride over the CTAs.
-                    const double *q = vpart + w * a.vgrid;
+                    const int cls = k % 3, r = k / 3;
                     double t = 0.0;
 #pragma unroll 1
-                    for (int k = 0; k < L::TEAMS && k * 32 < a.vgrid; ++k)
-                    {
-                        double s = 0.0;
-#pragma unroll 1
-                        for (int c = k * 32 + lane; c < a.vgrid; c += L::TEAMS * 32)
-                            s += q[c];
-                        t += warp_sum(s);
-                    }
+                    for (int c = r * 32 + lane; c < a.vgrid; c += L::TEAMS * 32)
+                        t += vpart[cls * a.vgrid + c];
+                    t = warp_sum(t);
                     if (lane == 0)
-                        sh.tot[w] = t;
+                        sh.tot[cls][r] = t;
                 }
                 __syncthreads();
                 if (tid == 0)
@@ -813,13 +943,19 @@ namespace pmas
                     if (init)
                         sh.st.rr0 = bank_total(sh.red + 8);
                     const double Lc = (double)a.cfg.level_num;
-                    sh.st.rz_coarse = sh.tot[2] + Lc * sh.tot[1];
+                    double tot[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+                    for (int r = 0; r < rounds; ++r)
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+                            tot[i] += sh.tot[i][r];
+                    sh.st.rz_coarse = tot[2] + Lc * tot[1];
                     sh.st.rzx_coarse = 0.0;
-                    pcg_finalize(&sh.st, a.cfg, init ? 1 : 2, sh.tot[0] + sh.tot[1] + sh.st.rz_coarse, 0.0);
+                    pcg_finalize(&sh.st, a.cfg, init ? 1 : 2, tot[0] + tot[1] + sh.st.rz_coarse, 0.0);
                 }
                 __syncthreads();
                 // ---- x += alpha p (unless the true residual's update did it) and p = z + beta p.
-                const bool pdo = !__shfl_sync(FULL, sh.st.done, 0), xdo = !residual;
+                const bool pdo = !warp_uniform(sh.st.done), xdo = !residual;
                 const double alpha = sh.st.alpha, beta = sh.st.beta;
                 const double iso_scale = 1.0 + mas.level_num;
 #pragma unroll 1
@@ -837,10 +973,10 @@ namespace pmas
                     {
                         if (k != w)
                             coarse_of(k);
-                        v += slot_next.x >= 0 ? zc_next[0] : 0.0;
-                        v += slot_next.y >= 0 ? zc_next[1] : 0.0;
-                        v += slot_next.z >= 0 ? zc_next[2] : 0.0;
-                        v += slot_next.w >= 0 ? zc_next[3] : 0.0;
+                        v += slot_next.x != 0xFFFF ? zc_next[0] : 0.0;
+                        v += slot_next.y != 0xFFFF ? zc_next[1] : 0.0;
+                        v += slot_next.z != 0xFFFF ? zc_next[2] : 0.0;
+                        v += slot_next.w != 0xFFFF ? zc_next[3] : 0.0;
                     }
                     else
                         v = iso_scale * v;
@@ -869,6 +1005,12 @@ namespace pmas
                 for (long long i = 0; i < MBAR_SPIN_LIMIT; ++i)
                     if (mbar_try_wait(&sh.bar, 0u))
                         break;
+#pragma unroll 1
+                for (int g = batch; g < batch + buffers; ++g)
+#pragma unroll 1
+                    for (long long i = 0; i < MBAR_SPIN_LIMIT; ++i)
+                        if (mbar_try_wait(&sh.ring_bar[g % buffers], (uint32_t)(g / buffers) & 1u))
+                            break;
                 if (!ok)
                 {
                     sh.st.error = ERR_TIMEOUT;
@@ -892,27 +1034,53 @@ namespace pmas
             const int sms = device_sm_count();
             const int items = mas.banks + mas.n_coarse_active;
             // The dots are summed as the iteration kernels do for one bank per warp of update_xr.
-            if (mas.level_num < 1 || mas.banks < 1 || mas.banks > PERSIST_MAX_BANKS ||
+            if (mas.level_num < 1 || mas.banks < 1 || mas.banks > (BD == 3 ? 2100 : (BD == 2 ? 3300 : 5200)) ||
                 update_xr_grid(mas) != (mas.banks + 7) / 8)
                 return pl;
             pl.vgrid = mas_apply_grid(mas);
             pl.teams = pl.vgrid * L::TEAMS;
             pl.busy = pl.teams < items ? pl.teams : items;
             pl.grid = pl.busy < sms ? pl.busy : sms;
-            pl.max_items = ((pl.busy + pl.grid - 1) / pl.grid) * ((items + pl.teams - 1) / pl.teams);
+            // The most items of a CTA (k_pcg_persistent's two divisions of the items).
+            const int nv = (pl.busy + pl.grid - 1) / pl.grid;
+            if (pl.busy == items)
+                for (int c = 0; c < pl.grid; ++c)
+                    pl.max_items =
+                        std::max(pl.max_items, (int)((long long)(c + 1) * mas.banks / pl.grid) -
+                                                   (int)((long long)c * mas.banks / pl.grid) +
+                                                   (mas.n_coarse_active - (pl.grid - 1 - c) + pl.grid - 1) / pl.grid);
+            else
+                for (int k = 0; k < items; k += pl.teams)
+                    pl.max_items += std::min(nv, (items - k + pl.grid - 1) / pl.grid);
             pl.deep_nodes = mas.real_count[1] + mas.real_count[2] + mas.real_count[3];
-            pl.staged = (((mas.banks + 7) & ~7) + 3 * pl.teams + 1) & ~1;
-            if (pl.deep_nodes < 0 || pl.deep_nodes > 1024 || mas.real_count[0] >= 0xFFFF)
+            const int extras = items - mas.first_iso_bank, team_dots = pl.busy + extras + 3;
+            pl.staged = (mas.banks + 7) / 8 * 9 + team_dots + team_dots / L::TEAMS + 2;
+            pl.staged += pl.staged & 1;
+            if (pl.deep_nodes < 0 || pl.deep_nodes > 1024 || mas.total_coarse * 32 >= 0xFFFF || extras > pl.teams)
                 return pl;
-            const size_t fixed = pl.max_items * (sizeof(ItemRec<BD>) + L::STAGE_BYTES) +
-                                 (size_t)PS_WARPS * PS_SCRATCH<BD, Store> +
+            const size_t fixed = pl.max_items * sizeof(ItemRec<BD>) + (size_t)PS_WARPS * PS_SCRATCH<BD, Store> +
                                  (size_t)((3 * pl.vgrid + 1) & ~1) * sizeof(double) +
                                  (size_t)((pl.deep_nodes * BD + 1) & ~1) * sizeof(double) +
                                  (size_t)pl.staged * sizeof(double) + (size_t)pl.deep_nodes * 64;
             if (fixed > PS_SMEM)
                 return pl;
-            pl.a_bytes = (int)((PS_SMEM - fixed) / 16 * 16);
-            pl.smem = fixed + pl.a_bytes;
+            const size_t room = PS_SMEM - fixed;
+            pl.slots = (int)std::min(room / L::STAGE_BYTES, (size_t)pl.max_items);
+            pl.batch = 1;
+            if (pl.slots < pl.max_items)
+            {
+                // Two buffers, each at most one round of the warps.
+                const int coarse = (mas.n_coarse_active + pl.grid - 1) / pl.grid + 1; // no CTA has more
+                pl.batch = std::min(PS_WARPS / BD, (pl.slots - coarse) / 2);
+                if (pl.batch < 1)
+                    return pl;
+                pl.ring = 2 * pl.batch;
+                const int rounds = (pl.max_items - (pl.slots - pl.ring) + pl.batch - 1) / pl.batch;
+                if (rounds > (std::is_same_v<Store, double> ? 11 : 7))
+                    return pl;
+            }
+            pl.a_bytes = (int)((room - (size_t)pl.slots * L::STAGE_BYTES) / 16 * 16);
+            pl.smem = fixed + (size_t)pl.slots * L::STAGE_BYTES + pl.a_bytes;
             pl.ok = true;
             return pl;
         }
@@ -935,11 +1103,14 @@ namespace pmas
         }
     } // namespace
 
-    // Every system whose inverses, vectors and coarse lists fit in the SMs' shared memory (290 banks of
-    // 96 x 96 FP64, 1,400 of FP16, 3,700 of 32 x 32): at each size measured up to there one launch was
-    // the faster path (the largest: 33^3 FP16 2,150 us against 3,060, 48^3 scalar FP16 3,930 against
-    // 4,250). Beyond, the inverses would stream from L2 through a ring: measured 1.2 to 2 times slower
-    // than the iteration kernels at 37^3 and 42^3.
+    // Where one launch is the faster path (us per solve_device, iteration kernels -> one launch). Inverses,
+    // vectors and coarse lists in shared memory: always (8^3 FP64 1,240 -> 640, 20^3 FP16 1,870 -> 910,
+    // 33^3 FP16 3,120 -> 1,830, 200 x 100 plane FP16 3,800 -> 1,830). Inverses through the ring: while
+    // few batches pass per apply and a CTA has at most some 14 banks of 96 rows (23 of 64, 35 of 32):
+    // 37^3 FP32 3,850 -> 2,690, 33^3 FP64 3,730 -> 2,640, 400 x 200 plane FP64 5,960 -> 4,700, 52^3 scalar
+    // FP64 5,040 -> 4,200. Beyond, both are alike and then the kernels faster: 42^3 FP16 4,250 -> 4,150,
+    // 42^3 FP32 (8 batches) 4,700 -> 5,300, 45^3 FP16 4,980 -> 5,700, 500 x 250 plane FP64 (13 batches)
+    // 7,100 -> 9,100, 56^3 scalar FP64 5,270 -> 5,270.
     PersistPlan persist_plan(const MasView &mas)
     {
         return dispatch_variant(mas.bd, mas.storage, [&]<int BD, class Store>() { return plan_variant<BD, Store>(mas); });
@@ -947,7 +1118,7 @@ namespace pmas
 
     size_t persist_dots_size(const MasView &mas, const PersistPlan &pl)
     {
-        return 2 * (size_t)((mas.banks + 7) & ~7) + (size_t)pl.staged;
+        return 3 * (size_t)((mas.banks + 7) & ~7) + (size_t)pl.busy + (mas.banks + mas.n_coarse_active - mas.first_iso_bank) + 4;
     }
 
     size_t persist_gather_size(const MasView &mas)
@@ -995,6 +1166,9 @@ namespace pmas
         a.vgrid = pl.vgrid;
         a.busy = pl.busy;
         a.max_items = pl.max_items;
+        a.slots = pl.slots;
+        a.ring = pl.ring;
+        a.batch = pl.batch;
         a.a_bytes = pl.a_bytes;
         a.deep_nodes = pl.deep_nodes;
         a.staged = pl.staged;

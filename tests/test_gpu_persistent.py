@@ -24,6 +24,10 @@ CASES = [
     (3, 20, "fp64", {}),
     (3, 24, "fp32", {"true_residual_period": 5, "ordering": "graph"}),
     (3, 33, "fp16", {"check_period": 1, "true_residual_period": 50}),
+    # inverses through the ring of bulk copies: two or three per batch, one per batch
+    (3, 38, "fp16", {"check_period": 1, "true_residual_period": 50, "max_iter": 45}),
+    (3, 36, "fp32", {"check_period": 1, "max_iter": 45}),
+    (3, 30, "fp64", {"check_period": 1, "max_iter": 45}),
     (2, 6, "fp64", {}),
     (2, 19, "fp32", {"ordering": "natural"}),
     (2, 22, "fp16", {"check_period": 1}),
