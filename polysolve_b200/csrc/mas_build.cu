@@ -657,6 +657,13 @@ namespace pmas
 
         int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+        // A copy in stream order, finished on return.
+        void copy_now(void *dst, const void *src, size_t bytes, cudaMemcpyKind kind, cudaStream_t s)
+        {
+            cuda_check(cudaMemcpyAsync(dst, src, bytes, kind, s), "copy");
+            cuda_check(cudaStreamSynchronize(s), "copy");
+        }
+
         template <class T>
         void exclusive_scan(const T *in, T *out, int n, cudaStream_t s)
         {
@@ -881,7 +888,7 @@ namespace pmas
                         k_fine_pair_count<<<div_up(nodes, 256), 256, 0, s>>>(A.view(), d_node_real, cnt.get());
                     cuda_check(cudaGetLastError(), "pair count launch");
                     exclusive_scan(cnt.get(), off.get(), nodes + 1, s);
-                    cuda_check(cudaMemcpy(&R, off.get() + nodes, sizeof(long long), cudaMemcpyDeviceToHost), "count");
+                    copy_now(&R, off.get() + nodes, sizeof(long long), cudaMemcpyDeviceToHost, s);
                     keys.alloc((size_t)std::max(R, 1LL), "MAS coarse_sums");
                     pay.alloc((size_t)std::max(R, 1LL), "MAS coarse_sums");
                     if (nodes > 0)
@@ -926,7 +933,7 @@ namespace pmas
                 cuda_check(cudaGetLastError(), "heads launch");
                 exclusive_scan(head.get(), hidx.get(), (int)R + 1, s);
                 int T = 0;
-                cuda_check(cudaMemcpy(&T, hidx.get() + R, sizeof(int), cudaMemcpyDeviceToHost), "targets");
+                copy_now(&T, hidx.get() + R, sizeof(int), cudaMemcpyDeviceToHost, s);
                 cs.ptr.alloc((size_t)T + 1, "MAS coarse_sums");
                 cs.pair.alloc((size_t)std::max(T, 1), "MAS coarse_sums");
                 k_key_targets<<<g1, 256, 0, s>>>(keys_s.get(), head.get(), hidx.get(), R, cn, cs.ptr.get(), cs.pair.get());
@@ -1070,7 +1077,7 @@ namespace pmas
         cuda_check(cudaGetLastError(), "cco lv0 launch");
         exclusive_scan(cnt.get(), M.cco0_base.get(), banks + 1, s);
         int C = 0;
-        cuda_check(cudaMemcpy(&C, M.cco0_base.get() + banks, sizeof(int), cudaMemcpyDeviceToHost), "count");
+        copy_now(&C, M.cco0_base.get() + banks, sizeof(int), cudaMemcpyDeviceToHost, s);
         k_map_lv0<<<div_up(nodes, 256), 256, 0, s>>>(nodes, M.lcco0.get(), M.cco0_base.get(), M.map.get());
         cuda_check(cudaGetLastError(), "map lv0 launch");
         for (int i = 0; i < MAX_COARSE; ++i)
@@ -1096,7 +1103,7 @@ namespace pmas
             cuda_check(cudaGetLastError(), "cco lvx launch");
             exclusive_scan(lcnt.get(), lbase.get(), cb + 1, s);
             int next = 0;
-            cuda_check(cudaMemcpy(&next, lbase.get() + cb, sizeof(int), cudaMemcpyDeviceToHost), "count");
+            copy_now(&next, lbase.get() + cb, sizeof(int), cudaMemcpyDeviceToHost, s);
             k_map_lvx<<<div_up(nodes, 256), 256, 0, s>>>(nodes, lv, lid.get(), lbase.get(), M.map.get());
             cuda_check(cudaGetLastError(), "map lvx launch");
             if (next == C)
@@ -1109,11 +1116,11 @@ namespace pmas
         if (M.level_num < MAX_COARSE)
         {
             std::vector<int> hmap((size_t)nodes * 4);
-            cuda_check(cudaMemcpy(hmap.data(), M.map.get(), hmap.size() * sizeof(int), cudaMemcpyDeviceToHost), "map");
+            copy_now(hmap.data(), M.map.get(), hmap.size() * sizeof(int), cudaMemcpyDeviceToHost, s);
             for (int u = 0; u < nodes; ++u)
                 for (int l = M.level_num; l < MAX_COARSE; ++l)
                     hmap[(size_t)u * 4 + l] = -1;
-            cuda_check(cudaMemcpy(M.map.get(), hmap.data(), hmap.size() * sizeof(int), cudaMemcpyHostToDevice), "map");
+            copy_now(M.map.get(), hmap.data(), hmap.size() * sizeof(int), cudaMemcpyHostToDevice, s);
         }
 
         // --- matrix counts and coarse vector layout
@@ -1145,7 +1152,7 @@ namespace pmas
             M.coff[l] = coff[l];
         {
             std::vector<int> hmap((size_t)nodes * 4);
-            cuda_check(cudaMemcpy(hmap.data(), M.map.get(), hmap.size() * sizeof(int), cudaMemcpyDeviceToHost), "map");
+            copy_now(hmap.data(), M.map.get(), hmap.size() * sizeof(int), cudaMemcpyDeviceToHost, s);
             std::vector<int> parent((size_t)cn, -1); // coarse node -> next-level coarse node
             for (int u = 0; u < nodes; ++u)
                 for (int l = 1; l < M.level_num; ++l)
@@ -1178,7 +1185,7 @@ namespace pmas
             if (fib < banks)
             {
                 std::vector<int> hreal((size_t)nodes);
-                cuda_check(cudaMemcpy(hreal.data(), d_node_real, sizeof(int) * nodes, cudaMemcpyDeviceToHost), "real");
+                copy_now(hreal.data(), d_node_real, sizeof(int) * nodes, cudaMemcpyDeviceToHost, s);
                 int rc_l[MAX_COARSE];
                 bool ok = true;
                 for (int l = 0; l < M.level_num && ok; ++l)

@@ -297,8 +297,44 @@ namespace
     std::atomic<bool> CooperativeTurn::taken[64];
 } // namespace
 
+namespace
+{
+    // The memory pool a handle factorizes with (AllocScope): freed temporaries of up to KEEP bytes stay in
+    // it for the next factorization, the rest and everything at the handle's end goes back to the device.
+    // Declared before the handle's buffers, so it is destroyed after them.
+    struct AllocPool
+    {
+        static constexpr uint64_t KEEP = 256ull << 20;
+        cudaMemPool_t pool = nullptr;
+        cudaMemPool_t get(int device)
+        {
+            if (pool)
+                return pool;
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            if (cudaMemPoolCreate(&pool, &props) != cudaSuccess)
+            {
+                cudaGetLastError();
+                pool = nullptr; // plain allocations then
+                return pool;
+            }
+            uint64_t keep = KEEP;
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            return pool;
+        }
+        ~AllocPool()
+        {
+            if (pool)
+                cudaMemPoolDestroy(pool);
+        }
+    };
+} // namespace
+
 struct mas_solver
 {
+    AllocPool alloc_pool;
     Params p;
     int device = 0;
     cudaStream_t own_stream = nullptr;
@@ -339,8 +375,10 @@ struct mas_solver
     std::vector<std::pair<std::string, double>> factorize_phases; // host-clock ms per phase
     DevBuf<double> refresh_vals; // CSC values on the device (kept: nnz doubles)
     // Pinned double buffer for large uploads from pageable host memory (the CSC values).
-    static constexpr size_t STAGE_BYTES = (size_t)16 << 20;
+    static constexpr size_t STAGE_BYTES = (size_t)16 << 20, STAGE_MIN = (size_t)4 << 20;
     char *h_stage = nullptr;
+    size_t stage_capacity = 0, stage_last = 0;
+    bool stage_used[2] = {false, false};
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};
     int launched_iterations = 0;
 
@@ -551,66 +589,97 @@ struct mas_solver
         cuda_check(cudaMallocHost(&h_st, 2 * sizeof(PcgState)), "pinned state");
     }
 
-    // Host -> device copy of a large pageable array: host threads copy 16 MB chunks into a pinned
-    // double buffer while the previous chunk's DMA runs (a plain pageable copy goes through one
-    // staging thread of the driver). Small arrays take the plain path.
+    // Chunk of a staged copy: an eighth of the array, within limits (both the host threads' copy and
+    // the DMA of a chunk then overlap with the others'). 0: too small to stage.
+    static size_t stage_chunk(size_t bytes)
+    {
+        if (bytes < STAGE_MIN)
+            return 0;
+        return std::min(STAGE_BYTES, std::max(STAGE_MIN / 4, (bytes / 8 + 4095) / 4096 * 4096));
+    }
+
+    // The pinned double buffer for chunks of `chunk` bytes. Uploads of an earlier array with chunks of
+    // another size may still be read from it: wait for them.
+    void ensure_stage(size_t chunk)
+    {
+        if (chunk != stage_last)
+            for (int slot = 0; slot < 2; ++slot)
+                if (stage_used[slot])
+                {
+                    cuda_check(cudaEventSynchronize(stage_ev[slot]), "staging");
+                    stage_used[slot] = false;
+                }
+        stage_last = chunk;
+        if (stage_capacity < 2 * chunk)
+        {
+            if (h_stage)
+                cudaFreeHost(h_stage);
+            h_stage = nullptr;
+            stage_capacity = 0;
+            cuda_check(cudaMallocHost(&h_stage, 2 * chunk), "pinned staging");
+            stage_capacity = 2 * chunk;
+        }
+        for (cudaEvent_t &e : stage_ev)
+            if (!e)
+                cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    }
+
+    static void parallel_copy(char *to, const char *from, size_t len, int threads)
+    {
+#pragma omp parallel for num_threads(threads) schedule(static)
+        for (int t = 0; t < threads; ++t)
+        {
+            const size_t a = len * t / threads, z = len * (t + 1) / threads;
+            std::memcpy(to + a, from + a, z - a);
+        }
+    }
+
+    // Host -> device copy of a large pageable array: host threads copy chunks into a pinned double
+    // buffer while the previous chunk's DMA runs (a plain pageable copy goes through one staging
+    // thread of the driver). Small arrays take the plain path. Returns with the last DMA in flight:
+    // `src` has been read.
     void upload_pageable(void *dst, const void *src, size_t bytes)
     {
-        if (bytes < 2 * STAGE_BYTES)
+        const size_t chunk = stage_chunk(bytes);
+        if (chunk == 0)
         {
             cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream), "upload");
             return;
         }
-        if (!h_stage)
-        {
-            cuda_check(cudaMallocHost(&h_stage, 2 * STAGE_BYTES), "pinned staging");
-            for (cudaEvent_t &e : stage_ev)
-                cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-        }
+        ensure_stage(chunk);
         const int threads = std::max(1, std::min(8, omp_get_max_threads()));
-        bool used[2] = {false, false};
-        for (size_t off = 0, i = 0; off < bytes; off += STAGE_BYTES, ++i)
+        for (size_t off = 0, i = 0; off < bytes; off += chunk, ++i)
         {
             const int slot = (int)(i & 1);
-            const size_t len = std::min(STAGE_BYTES, bytes - off);
-            if (used[slot])
+            const size_t len = std::min(chunk, bytes - off);
+            if (stage_used[slot])
                 cuda_check(cudaEventSynchronize(stage_ev[slot]), "staging");
-            char *buf = h_stage + slot * STAGE_BYTES;
-            const char *from = static_cast<const char *>(src) + off;
-#pragma omp parallel for num_threads(threads) schedule(static)
-            for (int t = 0; t < threads; ++t)
-            {
-                const size_t a = len * t / threads, z = len * (t + 1) / threads;
-                std::memcpy(buf + a, from + a, z - a);
-            }
+            char *buf = h_stage + slot * chunk;
+            parallel_copy(buf, static_cast<const char *>(src) + off, len, threads);
             cuda_check(cudaMemcpyAsync(static_cast<char *>(dst) + off, buf, len, cudaMemcpyHostToDevice, stream),
                        "upload");
             cuda_check(cudaEventRecord(stage_ev[slot], stream), "event");
-            used[slot] = true;
+            stage_used[slot] = true;
         }
     }
 
-    // Device -> host copy into pageable memory, the reverse of upload_pageable: 16 MB chunks DMA'd
-    // into the pinned double buffer while host threads copy the previous chunk out.
+    // Device -> host copy into pageable memory, the reverse of upload_pageable: chunks DMA'd into the
+    // pinned double buffer while host threads copy the previous chunk out.
     void download_pageable(void *dst, const void *src, size_t bytes)
     {
-        if (bytes < 2 * STAGE_BYTES)
+        const size_t chunk = stage_chunk(bytes);
+        if (chunk == 0)
         {
             cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream), "download");
             cuda_check(cudaStreamSynchronize(stream), "download");
             return;
         }
-        if (!h_stage)
-        {
-            cuda_check(cudaMallocHost(&h_stage, 2 * STAGE_BYTES), "pinned staging");
-            for (cudaEvent_t &e : stage_ev)
-                cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-        }
+        ensure_stage(chunk); // (stream order: earlier uploads have left the buffer before a download fills it)
         const int threads = std::max(1, std::min(8, omp_get_max_threads()));
-        const size_t chunks = (bytes + STAGE_BYTES - 1) / STAGE_BYTES;
+        const size_t chunks = (bytes + chunk - 1) / chunk;
         auto start = [&](size_t i) {
-            const size_t off = i * STAGE_BYTES, len = std::min(STAGE_BYTES, bytes - off);
-            cuda_check(cudaMemcpyAsync(h_stage + (i & 1) * STAGE_BYTES, static_cast<const char *>(src) + off, len,
+            const size_t off = i * chunk, len = std::min(chunk, bytes - off);
+            cuda_check(cudaMemcpyAsync(h_stage + (i & 1) * chunk, static_cast<const char *>(src) + off, len,
                                        cudaMemcpyDeviceToHost, stream),
                        "download");
             cuda_check(cudaEventRecord(stage_ev[i & 1], stream), "event");
@@ -621,15 +690,8 @@ struct mas_solver
             if (i + 1 < chunks)
                 start(i + 1); // stream order: chunk i + 1 goes into the other buffer
             cuda_check(cudaEventSynchronize(stage_ev[i & 1]), "staging");
-            const size_t off = i * STAGE_BYTES, len = std::min(STAGE_BYTES, bytes - off);
-            const char *buf = h_stage + (i & 1) * STAGE_BYTES;
-            char *to = static_cast<char *>(dst) + off;
-#pragma omp parallel for num_threads(threads) schedule(static)
-            for (int t = 0; t < threads; ++t)
-            {
-                const size_t a = len * t / threads, z = len * (t + 1) / threads;
-                std::memcpy(to + a, buf + a, z - a);
-            }
+            const size_t off = i * chunk, len = std::min(chunk, bytes - off);
+            parallel_copy(static_cast<char *>(dst) + off, h_stage + (i & 1) * chunk, len, threads);
         }
     }
 
@@ -650,6 +712,7 @@ struct mas_solver
             tp = now;
         };
         cuda_check(cudaSetDevice(device), "set device");
+        const AllocScope scope(alloc_pool.get(device), stream);
         if (declared)
         {
             if (!factorized)
@@ -760,10 +823,8 @@ struct mas_solver
                 DevBuf<int> d_outer, d_inner;
                 d_outer.alloc(n_ + 1, "MAS permuted_bsr input_csc");
                 d_inner.alloc(nnz_ > 0 ? nnz_ : 1, "MAS permuted_bsr input_csc");
-                cuda_check(cudaMemcpyAsync(d_outer.get(), outer, sizeof(int) * (n_ + 1), cudaMemcpyHostToDevice, stream),
-                           "upload outer");
-                cuda_check(cudaMemcpyAsync(d_inner.get(), inner, sizeof(int) * nnz_, cudaMemcpyHostToDevice, stream),
-                           "upload inner");
+                upload_pageable(d_outer.get(), outer, sizeof(int) * (size_t)(n_ + 1));
+                upload_pageable(d_inner.get(), inner, sizeof(int) * (size_t)nnz_);
                 A.slice.reset();
                 A.cols.reset();
                 A.vals.reset();

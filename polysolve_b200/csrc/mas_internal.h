@@ -50,8 +50,23 @@ namespace pmas
     };
 
     void cuda_check(cudaError_t e, const char *what);
-    void *device_alloc(size_t bytes, const char *ctx); // throws Error(ERR_OOM) with MB figures
-    void device_free(void *p);
+    // Stream-ordered allocation for the calling thread while an AllocScope lives: buffers come from
+    // the scope's memory pool in the order of its stream, and buffers that did return to it the same
+    // way, without the device-wide synchronisation of cudaFree. Work on the memory inside the scope
+    // has to be on that stream.
+    struct AllocScope
+    {
+        cudaMemPool_t saved_pool;
+        cudaStream_t saved_stream;
+        AllocScope(cudaMemPool_t pool, cudaStream_t s);
+        ~AllocScope();
+        AllocScope(const AllocScope &) = delete;
+        AllocScope &operator=(const AllocScope &) = delete;
+    };
+
+    // throws Error(ERR_OOM) with MB figures; *pooled: the memory came from the thread's AllocScope
+    void *device_alloc(size_t bytes, const char *ctx, bool *pooled);
+    void device_free(void *p, bool pooled);
     // Test hook: after `after` more successful device allocations the next one fails as if the
     // device were out of memory (once); negative: off.
     void set_alloc_failure(long long after);
@@ -62,6 +77,7 @@ namespace pmas
     {
         T *p = nullptr;
         size_t n = 0;
+        bool pooled = false;
         DevBuf() = default;
         DevBuf(const DevBuf &) = delete;
         DevBuf &operator=(const DevBuf &) = delete;
@@ -69,7 +85,7 @@ namespace pmas
         void reset()
         {
             if (p)
-                device_free(p);
+                device_free(p, pooled);
             p = nullptr;
             n = 0;
         }
@@ -79,7 +95,7 @@ namespace pmas
                 return;
             reset();
             if (count)
-                p = static_cast<T *>(device_alloc(count * sizeof(T), ctx));
+                p = static_cast<T *>(device_alloc(count * sizeof(T), ctx, &pooled));
             n = count;
         }
         T *get() const { return p; }

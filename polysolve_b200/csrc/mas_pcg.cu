@@ -32,10 +32,26 @@ namespace pmas
 
     void set_alloc_failure(long long after) { g_alloc_fail_after.store(after < 0 ? -1 : after); }
 
+    static thread_local cudaMemPool_t t_alloc_pool = nullptr;
+    static thread_local cudaStream_t t_alloc_stream = nullptr;
+
+    AllocScope::AllocScope(cudaMemPool_t pool, cudaStream_t s) : saved_pool(t_alloc_pool), saved_stream(t_alloc_stream)
+    {
+        t_alloc_pool = pool;
+        t_alloc_stream = s;
+    }
+
+    AllocScope::~AllocScope()
+    {
+        t_alloc_pool = saved_pool;
+        t_alloc_stream = saved_stream;
+    }
+
     // Allocation with the reference's out-of-memory message (mas_utils/CudaUtils.cuh:68-79).
-    void *device_alloc(size_t bytes, const char *ctx)
+    void *device_alloc(size_t bytes, const char *ctx, bool *pooled)
     {
         void *p = nullptr;
+        *pooled = t_alloc_pool != nullptr;
         cudaError_t e = cudaErrorMemoryAllocation;
         long long left = g_alloc_fail_after.load();
         bool injected = false;
@@ -49,7 +65,7 @@ namespace pmas
             }
         }
         if (!injected)
-            e = cudaMalloc(&p, bytes);
+            e = *pooled ? cudaMallocFromPoolAsync(&p, bytes, t_alloc_pool, t_alloc_stream) : cudaMalloc(&p, bytes);
         if (e == cudaSuccess)
             return p;
         if (e != cudaErrorMemoryAllocation)
@@ -63,9 +79,13 @@ namespace pmas
                                  std::to_string(free_b / mb) + " MB free.");
     }
 
-    void device_free(void *p)
+    void device_free(void *p, bool pooled)
     {
-        if (p)
+        if (!p)
+            return;
+        if (pooled && t_alloc_pool)
+            cudaFreeAsync(p, t_alloc_stream);
+        else
             cudaFree(p);
     }
 
