@@ -427,16 +427,28 @@ namespace pmas
             pdl_release(); // this warp's items are done: the successor may start launching
             if (MODE == 0)
                 return;
-            double tot[APPLY_PARTS];
-            if (grid_reduce<APPLY_PARTS, THREADS, L::TEAMS * 32>(part, red.rz_parts, &st->counter[4], tot, cta) &&
-                threadIdx.x == 0)
+            // Isolated rows: z = (1 + L) z0, so their r.z is (1 + L) r.z0 -- r.z0 is in the
+            // level-0 sums, the coarse levels add L r.z0.
+            const double Lc = (double)cfg.level_num;
+            // (The dots with the previous z are wanted, and formed, for Polak-Ribiere's beta only.)
+            if (MODE == 2 && cfg.polak_ribiere)
             {
-                // Isolated rows: z = (1 + L) z0, so their r.z is (1 + L) r.z0 -- r.z0 is in the
-                // level-0 sums, the coarse levels add L r.z0.
-                const double Lc = (double)cfg.level_num;
-                st->rz_coarse = tot[4] + Lc * tot[2];
-                st->rzx_coarse = tot[5] + Lc * tot[3];
-                pcg_finalize(st, cfg, MODE, tot[0] + tot[2] + st->rz_coarse, tot[1] + tot[3] + st->rzx_coarse);
+                double tot[APPLY_PARTS];
+                if (grid_reduce<APPLY_PARTS, THREADS, L::TEAMS * 32>(part, red.rz_parts, &st->counter[4], tot, cta) &&
+                    threadIdx.x == 0)
+                {
+                    st->rz_coarse = tot[4] + Lc * tot[2];
+                    st->rzx_coarse = tot[5] + Lc * tot[3];
+                    pcg_finalize(st, cfg, MODE, tot[0] + tot[2] + st->rz_coarse, tot[1] + tot[3] + st->rzx_coarse);
+                }
+                return;
+            }
+            double rz[3] = {part[0], part[2], part[4]}, tot[3];
+            if (grid_reduce<3, THREADS, L::TEAMS * 32>(rz, red.rz_parts, &st->counter[4], tot, cta) && threadIdx.x == 0)
+            {
+                st->rz_coarse = tot[2] + Lc * tot[1];
+                st->rzx_coarse = 0.0;
+                pcg_finalize(st, cfg, MODE, tot[0] + tot[1] + st->rz_coarse, 0.0);
             }
         }
 
