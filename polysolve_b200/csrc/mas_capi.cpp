@@ -551,8 +551,9 @@ struct mas_solver
     void apply_levels(const MasView &mv, const PcgConfig &cfg, int mode)
     {
         PcgState *S = st.get();
-        run("coarse_levels", 0, [&] { return launch_coarse_levels(mv, S, stream); });
-        run("mas_apply", 1, [&] { launch_mas_apply(mv, r.get(), z.get(), S, red(), cfg, mode, stream); });
+        int levels = 0;
+        run("coarse_levels", 0, [&] { return levels = launch_coarse_levels(mv, S, stream); });
+        run("mas_apply", 1, [&] { launch_mas_apply(mv, r.get(), z.get(), S, red(), cfg, mode, levels > 0, stream); });
     }
 
     void collect_profile()
@@ -3079,7 +3080,7 @@ extern "C" int mas_debug_apply(mas_solver *h, const double *rin, double *zout, i
         const MasView mv = h->mas.view();
         launch_restrict(mv, h->r.get(), nullptr, 0, h->stream);
         launch_coarse_levels(mv, nullptr, h->stream);
-        launch_mas_apply(mv, h->r.get(), h->z.get(), nullptr, h->red(), h->config(), 0, h->stream);
+        launch_mas_apply(mv, h->r.get(), h->z.get(), nullptr, h->red(), h->config(), 0, false, h->stream);
         launch_prolong(mv, h->z.get(), h->Ap.get(), h->stream);
         cuda_check(cudaMemcpyAsync(zout, h->Ap.get(), sizeof(double) * len, cudaMemcpyDeviceToHost, h->stream), "z");
         cuda_check(cudaStreamSynchronize(h->stream), "apply");

@@ -455,9 +455,10 @@ namespace pmas
     // Coarse levels >= 2 summed from the first coarse level; returns the number of kernels launched.
     int launch_coarse_levels(const MasView &mas, const PcgState *st, cudaStream_t s);
     // z0 = A_0^-1 r and zc = A_l^-1 rc for all coarse levels (rc must be complete); mode 1 / 2 also
-    // run the PCG scalar step in the last CTA (1: initial apply, 2: iteration).
+    // run the PCG scalar step in the last CTA (1: initial apply, 2: iteration). after_levels: the launch
+    // before this one in the stream is launch_coarse_levels' kernel.
     void launch_mas_apply(const MasView &mas, const double *r, double *z0, PcgState *st, ReduceBuf red,
-                          PcgConfig cfg, int mode, cudaStream_t s);
+                          PcgConfig cfg, int mode, bool after_levels, cudaStream_t s);
     void launch_prolong(const MasView &mas, const double *z0, double *z, cudaStream_t s);
     // Grids of one system's restrict, coarse-level and apply launches (0: none), and the
     // batched launches (mode 1 / 2 applies only).
