@@ -410,6 +410,7 @@ struct mas_solver
     DevBuf<double> persist_dots, persist_gather;
     DevBuf<unsigned> persist_bar;
     bool persist_ready = false;
+    double l2_bytes = 0.0;
     bool in_batch = false; // solving as one of several systems of mas_solve_batch
 
     // Several right-hand sides at once: groups of RHS_GROUP interleaved vectors, one PcgState
@@ -588,6 +589,9 @@ struct mas_solver
         cuda_check(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking), "stream create");
         stream = own_stream;
         cuda_check(cudaMallocHost(&h_st, 2 * sizeof(PcgState)), "pinned state");
+        int l2 = 0;
+        if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device) == cudaSuccess)
+            l2_bytes = l2;
     }
 
     // Chunk of a staged copy: an eighth of the array, within limits (both the host threads' copy and
@@ -943,6 +947,23 @@ struct mas_solver
         return c;
     }
 
+    // Banks of the matrix that stay in L2 from one SpMV to the next: what fits beside the iteration's
+    // vectors (x, r, p, Ap, z and the coarse slots) in 7/16 of the L2, for the halves of the chip
+    // keep copies of what both read. The others are read past them, evict-first. Of 126 MB, with
+    // 0 / 20 / 30 / 40 / 50 MB kept, an iteration takes 48.0 / 45.6 / 44.1 / 43.2 / 44.6 us at 44^3 (binary16,
+    // the rule: 45 MB), 123.8 / 120.7 / 121.8 / 124.8 / 128.6 us at 61^3 (FP64, 25 MB), 43.1 / 42.4 / 40.5 /
+    // 41.9 / 39.9 us on a 500 x 500 plane (FP64, 32 MB), and at 80^3, whose vectors fill the L2, 172.5 /
+    // 174.3 us with 0 / 20. (A share of every 32 banks: 45.5 us at 44^3 for 40 MB.) Not in a batch,
+    // whose systems share the L2.
+    int kept_banks() const
+    {
+        const double room = l2_bytes * (7.0 / 16.0) - 5.0 * x.bytes() - 16.0 * 32.0 * banks;
+        const double matrix = (double)A.vals.bytes() + (double)A.cols.bytes();
+        if (in_batch || room <= 0.0 || matrix <= 0.0)
+            return 0;
+        return (int)(banks * std::min(1.0, room / matrix));
+    }
+
     // One PCG iteration's kernels (MASSolver.cu:498-583). residual: launch the true-residual SpMV
     // and its restriction (both check (st->iter + 1) % P == 0 on the device and return at once
     // otherwise; update_xr restricts r on the other iterations).
@@ -1027,6 +1048,7 @@ struct mas_solver
         mix((uint64_t)chained_launch());
         mix((uint64_t)spmv_unroll());
         mix((uint64_t)apply_items_per_warp());
+        mix((uint64_t)Av.keep);
         uint64_t bits;
         std::memcpy(&bits, &cfg.rel_tol, 8);
         mix(bits);
@@ -1077,7 +1099,8 @@ struct mas_solver
     // pcg_solve (MASSolver.cu:469-595) on device-resident b_ / x_ (padded order).
     void pcg()
     {
-        const BankedView Av = A.view();
+        BankedView Av = A.view();
+        Av.keep = kept_banks();
         const MasView mv = mas.view();
         const PcgConfig cfg = config();
         cudaEvent_t e0, e1;

@@ -388,6 +388,13 @@ namespace pmas
         return pol;
     }
 
+    __device__ __forceinline__ uint64_t l2_evict_normal_policy()
+    {
+        uint64_t pol;
+        asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+        return pol;
+    }
+
     __device__ __forceinline__ void bulk_load_stream(void *dst, const void *src, uint32_t bytes, uint64_t *bar,
                                                      uint64_t policy)
     {

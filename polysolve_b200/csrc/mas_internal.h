@@ -118,6 +118,7 @@ namespace pmas
         const int *rowlen;      // nodes
         const int *cols;        // slots * 32, padded node ids
         const double *vals;     // slots * 32 * bd * bd
+        int keep = 0;           // banks below it stay in L2 between products, the others stream through
     };
 
     __host__ __device__ inline long long banked_value_index(long long slot, int lane, int q, int bd)

@@ -61,8 +61,9 @@ namespace pmas
                 for (int i = 0; i < BD; ++i)
                     acc[i] = 0.0;
                 // The matrix streams through L2 with evict-first priority (x, the gathered vector,
-                // and the other PCG vectors stay resident); two slots' loads in flight per lane.
-                const uint64_t pol = l2_evict_first_policy();
+                // and the other PCG vectors stay resident), but for its first A.keep banks where the
+                // vectors leave room (kept_banks); two slots' loads in flight per lane.
+                const uint64_t pol = bank < A.keep ? l2_evict_normal_policy() : l2_evict_first_policy();
                 if constexpr (BD == 1 && UNROLL > 1)
                 {
                     // Scalar rows: four times as many slots for the same bytes in flight, and the last
