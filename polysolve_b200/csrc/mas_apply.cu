@@ -1386,103 +1386,72 @@ namespace pmas
         }
 
         // The coarse levels for nodes of NC components (the wide groups: 3 components x 16 right-hand
-        // sides), the same sums as k_coarse_levels in chunks of CH components, so the registers do not
-        // grow with NC.
-        template <int NC, int CH>
-        __device__ __forceinline__ void kid_sum_chunk(const MasView &mas, int l, int i, bool cg, int c0,
-                                                      double (&v)[CH])
-        {
-            const int lane = threadIdx.x & 31;
-            const int b = mas.kid_ptr[l][i], e = mas.kid_ptr[l][i + 1];
-#pragma unroll
-            for (int c = 0; c < CH; ++c)
-                v[c] = 0.0;
-            if (b + lane < e)
-            {
-                const size_t node = (size_t)mas.coff[l - 1] + mas.kids[b + lane];
-#pragma unroll
-                for (int c = 0; c < CH; ++c)
-                    v[c] = cg ? __ldcg(mas.rc + node * NC + c0 + c) : mas.rc[node * NC + c0 + c];
-            }
-#pragma unroll
-            for (int c = 0; c < CH; ++c)
-                v[c] = warp_sum(v[c]);
-        }
+        // sides): a thread per component of a node, whose 32 children's values, consecutive over the
+        // threads, are all on their way at once and are added in warp_sum's order (the bits of
+        // k_coarse_levels). Level 1 over the device, the few nodes above it in the last CTA to finish. A
+        // warp per node and eight components at a time, two warp sums in a row per value, took 40 us
+        // at 40^3 in three CTAs, now 16 us (both with about 6 us of the timing events).
+        constexpr int LEVEL_C_NODES = 4; // nodes of a CTA at a time
 
-        template <int NC, int CH>
-        __global__ void __launch_bounds__(LEVEL_THREADS) k_coarse_levels_c(MasView mas, const PcgState *grp)
+        template <int NC>
+        __device__ __forceinline__ void kid_sums(const MasView &mas, int l, int i0, int count,
+                                                 int (&kid)[LEVEL_C_NODES][32])
         {
-            static_assert(NC % CH == 0, "whole chunks");
-            if (grp && grp->done)
-                return;
-            constexpr int W = LEVEL_THREADS / 32;
-            const int w = warp_index(), lane = threadIdx.x & 31;
-            __shared__ double part[W][NC];
-            __shared__ int is_last;
-            if (mas.level_num == 2)
+            __syncthreads(); // the previous nodes' indices are done with; their sums are written
+            for (int q = threadIdx.x; q < LEVEL_C_NODES * 32; q += LEVEL_C_NODES * NC)
             {
-                const int i = blockIdx.x * W + w;
-                if (i >= mas.real_count[1])
-                    return;
-                for (int c0 = 0; c0 < NC; c0 += CH)
+                const int i = i0 + q / 32;
+                int node = -1;
+                if (i < count)
                 {
-                    double v[CH];
-                    kid_sum_chunk<NC, CH>(mas, 1, i, false, c0, v);
-                    if (lane == 0)
-#pragma unroll
-                        for (int c = 0; c < CH; ++c)
-                            mas.rc[((size_t)mas.coff[1] + i) * NC + c0 + c] = v[c];
+                    const int b = mas.kid_ptr[l][i], e = mas.kid_ptr[l][i + 1];
+                    if (b + q % 32 < e)
+                        node = mas.coff[l - 1] + mas.kids[b + q % 32];
                 }
-                return;
-            }
-            const int j = blockIdx.x;
-            const int kb = warp_uniform(mas.kid_ptr[2][j]), ke = warp_uniform(mas.kid_ptr[2][j + 1]);
-            if (kb + w < ke)
-            {
-                const int i = mas.kids[kb + w];
-                for (int c0 = 0; c0 < NC; c0 += CH)
-                {
-                    double v[CH];
-                    kid_sum_chunk<NC, CH>(mas, 1, i, false, c0, v);
-                    if (lane == 0)
-#pragma unroll
-                        for (int c = 0; c < CH; ++c)
-                        {
-                            mas.rc[((size_t)mas.coff[1] + i) * NC + c0 + c] = v[c];
-                            part[w][c0 + c] = v[c];
-                        }
-                }
+                kid[q / 32][q % 32] = node;
             }
             __syncthreads();
-            // The level-2 node's components, one per warp (in the same order as one warp would sum them).
-            for (int c = w; c < NC; c += W)
+            const int k = threadIdx.x / NC, c = threadIdx.x - k * NC;
+            if (i0 + k >= count)
+                return;
+            double v[32];
+#pragma unroll
+            for (int q = 0; q < 32; ++q)
             {
-                const double t = warp_sum(kb + lane < ke ? part[lane][c] : 0.0);
-                if (lane == 0)
-                    mas.rc[((size_t)mas.coff[2] + j) * NC + c] = t;
+                const int node = kid[k][q];
+                v[q] = node >= 0 ? __ldcg(mas.rc + (size_t)node * NC + c) : 0.0;
             }
-            if (mas.level_num <= 3)
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1)
+#pragma unroll
+                for (int q = 0; q < o; ++q)
+                    v[q] += v[q + o];
+            mas.rc[((size_t)mas.coff[l] + i0 + k) * NC + c] = v[0];
+        }
+
+        template <int NC>
+        __global__ void __launch_bounds__(LEVEL_C_NODES *NC) k_coarse_levels_c(MasView mas, const PcgState *grp)
+        {
+            if (grp && grp->done)
+                return;
+            __shared__ int kid[LEVEL_C_NODES][32];
+            __shared__ int is_last;
+            kid_sums<NC>(mas, 1, blockIdx.x * LEVEL_C_NODES, mas.real_count[1], kid);
+            if (mas.level_num <= 2)
                 return;
             __syncthreads();
             if (threadIdx.x == 0)
             {
-                __threadfence();
+                __threadfence(); // cumulative: orders this CTA's stores (seen at the barrier) first
                 is_last = atomicAdd(mas.ticket, 1u) == gridDim.x - 1;
             }
             __syncthreads();
             if (!warp_uniform(is_last))
                 return;
             __threadfence();
-            for (int k = w; k < mas.real_count[3]; k += W)
-                for (int c0 = 0; c0 < NC; c0 += CH)
-                {
-                    double v[CH];
-                    kid_sum_chunk<NC, CH>(mas, 3, k, true, c0, v);
-                    if (lane == 0)
-#pragma unroll
-                        for (int c = 0; c < CH; ++c)
-                            mas.rc[((size_t)mas.coff[3] + k) * NC + c0 + c] = v[c];
-                }
+            for (int l = 2; l < mas.level_num && l <= 3; ++l)
+                for (int i0 = 0; i0 < mas.real_count[l]; i0 += LEVEL_C_NODES)
+                    kid_sums<NC>(mas, l, i0, mas.real_count[l], kid);
             if (threadIdx.x == 0)
                 *mas.ticket = 0u;
         }
@@ -1814,11 +1783,8 @@ namespace pmas
     {
         if (mas.level_num <= 1 || mas.real_count[1] <= 0)
             return 0;
-        const int grid = mas.level_num == 2 ? (mas.real_count[1] + LEVEL_THREADS / 32 - 1) / (LEVEL_THREADS / 32)
-                                            : mas.real_count[2];
-        if (grid <= 0)
-            return 0;
-        k_coarse_levels_c<3 * RHS_WIDE, 8><<<grid, LEVEL_THREADS, 0, s>>>(mas, grp);
+        const int grid = (mas.real_count[1] + LEVEL_C_NODES - 1) / LEVEL_C_NODES;
+        k_coarse_levels_c<3 * RHS_WIDE><<<grid, LEVEL_C_NODES * 3 * RHS_WIDE, 0, s>>>(mas, grp);
         cuda_check(cudaGetLastError(), "wide coarse levels launch");
         return 1;
     }
