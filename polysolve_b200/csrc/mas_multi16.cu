@@ -337,6 +337,11 @@ namespace pmas
         }
 
         constexpr int XR_SMEM = WW * 32 * VN * 8; // per-warp component sums (96 KB per CTA)
+        // Steps of 32 values on their way in update_xr: 16 warps per SM (the sums' shared memory) with a
+        // bank each, so latency counts. In turns of four steps, 24.7 us at 40^3 (with about 6 us of the
+        // timing events); eight and the next eight, 23.0 us.
+        constexpr int STEP = 8;
+        static_assert(VN % STEP == 0, "whole steps");
 
         __global__ void __launch_bounds__(WT_) k_update_xr_w(MasView mas, double *__restrict__ x,
                                                              double *__restrict__ r, const double *__restrict__ p,
@@ -362,32 +367,44 @@ namespace pmas
                 int lc = -1, ncco = 0;
                 if (rs)
                     ncco = restrict_begin(mas, bank, acc, lc);
-                for (int t0 = 0; t0 < VN; t0 += 4)
-                {
-                    double xv[4], pv[4], av[4], rv[4];
+                // The next step's loads (Ap and r, or x and p) are on their way during this one's sums.
+                double na[STEP], nb[STEP];
+                auto load = [&](int t0) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < STEP; ++j)
                     {
                         const long long e = b0 + (t0 + j) * 32 + lane;
-                        xv[j] = due ? x[e] : 0.0;
-                        pv[j] = due ? p[e] : 0.0;
-                        av[j] = due ? 0.0 : Ap[e];
-                        rv[j] = due ? 0.0 : r[e];
+                        na[j] = due ? x[e] : Ap[e];
+                        nb[j] = due ? p[e] : r[e];
                     }
+                };
+                load(0);
+                for (int t0 = 0; t0 < VN; t0 += STEP)
+                {
+                    double av[STEP], bv[STEP];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < STEP; ++j)
+                    {
+                        av[j] = na[j];
+                        bv[j] = nb[j];
+                    }
+                    if (t0 + STEP < VN)
+                        load(t0 + STEP);
+#pragma unroll
+                    for (int j = 0; j < STEP; ++j)
                     {
                         const int el = (t0 + j) * 32 + lane;
+                        double rv = 0.0;
                         if (due)
-                            x[b0 + el] = fma(a, pv[j], xv[j]);
-                        if (!due)
+                            x[b0 + el] = fma(a, bv[j], av[j]);
+                        else
                         {
-                            rv[j] = fma(-a, av[j], rv[j]);
-                            r[b0 + el] = rv[j];
-                            part = fma(rv[j], rv[j], part);
+                            rv = fma(-a, av[j], bv[j]);
+                            r[b0 + el] = rv;
+                            part = fma(rv, rv, part);
                         }
                         if (rs)
-                            restrict_add(acc, lc, el, rv[j]);
+                            restrict_add(acc, lc, el, rv);
                     }
                 }
                 if (rs)
@@ -442,7 +459,12 @@ namespace pmas
             }
         }
 
-        // p_g = z0_g + sum_l zc_g[cslot_l(node)] + beta_g p_g (first: p = z); a warp per bank.
+        // p_g = z0_g + sum_l zc_g[cslot_l(node)] + beta_g p_g (first: p = z); a warp per third of a bank
+        // (a warp per bank left an SM 15 warps at 40^3, each with 12 rounds of two latencies: 32.8 us with
+        // about 6 us of the timing events; now P_W_US).
+        constexpr int P_PARTS = 3;
+        static_assert(VN % (4 * P_PARTS) == 0, "whole rounds");
+
         __global__ void __launch_bounds__(WT_) k_update_p_w(MasView mas, double *__restrict__ x,
                                                             double *__restrict__ p,
                                                             const double *__restrict__ z0, const PcgState *st,
@@ -454,7 +476,8 @@ namespace pmas
             if (grp->done && !xdo)
                 return;
             const int lane = threadIdx.x & 31;
-            const int bank = blockIdx.x * WW + warp_index();
+            const int item = blockIdx.x * WW + warp_index();
+            const int bank = item / P_PARTS, t_first = (item - bank * P_PARTS) * (VN / P_PARTS);
             if (bank >= mas.banks)
                 return;
             const int g = lane & (G - 1);
@@ -465,7 +488,7 @@ namespace pmas
             const double iso_scale = 1.0 + mas.level_num;
             const bool iso = bank >= mas.first_iso_bank;
             const long long b0 = (long long)bank * 32 * VN;
-            for (int t0 = 0; t0 < VN; t0 += 4)
+            for (int t0 = t_first; t0 < t_first + VN / P_PARTS; t0 += 4)
             {
                 double zv[4], po[4], xv[4];
                 int4 cs[4];
@@ -614,7 +637,7 @@ namespace pmas
     void launch_update_p_w(const MasView &mas, double *x, double *p, const double *z0, PcgState *st, int first,
                            cudaStream_t s)
     {
-        const int grid = (mas.banks + WW - 1) / WW;
+        const int grid = (mas.banks * P_PARTS + WW - 1) / WW;
         if (grid > 0)
             k_update_p_w<<<grid, WT_, 0, s>>>(mas, x, p, z0, st, first);
         cuda_check(cudaGetLastError(), "wide update_p launch");
