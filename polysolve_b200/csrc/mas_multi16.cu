@@ -461,7 +461,7 @@ namespace pmas
 
         // p_g = z0_g + sum_l zc_g[cslot_l(node)] + beta_g p_g (first: p = z); a warp per third of a bank
         // (a warp per bank left an SM 15 warps at 40^3, each with 12 rounds of two latencies: 32.8 us with
-        // about 6 us of the timing events; now P_W_US).
+        // about 6 us of the timing events, now 26.4 us).
         constexpr int P_PARTS = 3;
         static_assert(VN % (4 * P_PARTS) == 0, "whole rounds");
 
