@@ -23,7 +23,8 @@ namespace pmas
     // Programmatic dependent launch. The PCG iteration kernels are launched with programmatic
     // stream serialization (launch_chained): such a kernel may become resident while its
     // predecessor in the stream drains, so it calls pdl_wait() before it reads or writes anything
-    // that the predecessor (or any earlier kernel) touches. pdl_wait() returns once the
+    // that the predecessor (or any earlier kernel) touches (the apply beside k_coarse_levels
+    // excepted, see mas_apply_body). pdl_wait() returns once the
     // predecessor grid has completed and its writes are visible, and at once for a kernel
     // launched without the attribute. pdl_release() lets the successor start launching once every
     // CTA of this grid has called it or exited; it does not make any write visible early.

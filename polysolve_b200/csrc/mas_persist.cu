@@ -1026,6 +1026,21 @@ namespace pmas
         constexpr size_t PS_SMEM = 232448 - 1024; // dynamic shared memory beside the static part
         static_assert(sizeof(PsShared) <= 1024, "static shared memory of the persistent solve");
 
+        // Banks up to which one launch is the faster way: beyond, an SM's 12 warps are busy with products
+        // for longer than the iteration kernels' launches cost. us per iteration, one launch / iteration
+        // kernels, on both sides of each line: 3 x 3 blocks FP64 38.5 / 39.9 at 1,350 banks and 42.8 / 40.1
+        // at 1,470, FP32 36.1 / 41.5 at 1,716 and 43.3 / 42.4 at 1,855, binary16 29.6 / 36.6 at 1,584 and
+        // 37.4 / 37.3 at 1,855; 2 x 2 FP64 26.0 / 28.6 at 1,670 and 30.5 / 29.8 at 1,930, FP32 27.6 / 27.7 at
+        // 2,220 and 31.5 / 30.1 at 2,519, binary16 28.2 / 28.4 at 2,519; scalar FP64 23.7 / 25.8 at 3,050 and
+        // 28.6 / 26.5 at 3,680, FP32 and binary16 28.2 / 29.2 and 28.1 / 28.7 at 4,930.
+        template <int BD, class Store>
+        constexpr int persist_max_banks()
+        {
+            if (std::is_same_v<Store, double>)
+                return BD == 3 ? 1400 : (BD == 2 ? 1800 : 3200);
+            return BD == 3 ? (std::is_same_v<Store, float> ? 1800 : 1900) : (BD == 2 ? 2300 : PERSIST_MAX_BANKS);
+        }
+
         template <int BD, class Store>
         PersistPlan plan_variant(const MasView &mas)
         {
@@ -1034,7 +1049,7 @@ namespace pmas
             const int sms = device_sm_count();
             const int items = mas.banks + mas.n_coarse_active;
             // The dots are summed as the iteration kernels do for one bank per warp of update_xr.
-            if (mas.level_num < 1 || mas.banks < 1 || mas.banks > (BD == 3 ? 2100 : (BD == 2 ? 3300 : 5200)) ||
+            if (mas.level_num < 1 || mas.banks < 1 || mas.banks > persist_max_banks<BD, Store>() ||
                 update_xr_grid(mas) != (mas.banks + 7) / 8)
                 return pl;
             pl.vgrid = mas_apply_grid(mas);
@@ -1076,7 +1091,7 @@ namespace pmas
                     return pl;
                 pl.ring = 2 * pl.batch;
                 const int rounds = (pl.max_items - (pl.slots - pl.ring) + pl.batch - 1) / pl.batch;
-                if (rounds > (std::is_same_v<Store, double> ? 11 : 7))
+                if (rounds > 7)
                     return pl;
             }
             pl.a_bytes = (int)((room - (size_t)pl.slots * L::STAGE_BYTES) / 16 * 16);

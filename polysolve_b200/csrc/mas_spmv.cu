@@ -21,7 +21,7 @@ namespace pmas
         constexpr int BANKS_PER_CTA = SPMV_THREADS / 32;
 
         // UNROLL slots per loop trip, their loads in flight together (the spmv_unroll parameter:
-        // 1, 2 or 4; 2 measured best at 1.6 M DOF). Minimum one CTA per SM: the compiler then keeps
+        // 1, 2 or 4; 2 measured best at 1.6 M DOF; scalar rows take four times as many from 2 on). Minimum one CTA per SM: the compiler then keeps
         // the unrolled slots' loads in flight (80 registers at 2, 3 CTAs per SM), measured faster
         // than the occupancy-first 44-register build at 1.6 M DOF.
         template <int BD, int MODE, int UNROLL>
