@@ -21,7 +21,7 @@
 // team m mod (grid * teams per CTA) -- for r.z). Each CTA computes all totals and the scalar step
 // itself.
 //
-// Measured: persist_plan below. An iteration at 20^3 is some 29,000 cycles: four barriers of 2,400 (148
+// Measured: persist_max_banks below. An iteration at 20^3 is some 29,000 cycles: four barriers of 2,400 (148
 // CTAs), 3,500 for the SpMV (one round of gathers from L2), 4,500 for the totals and the scalar step,
 // 5,000 for the coarse levels.
 
@@ -1118,14 +1118,10 @@ namespace pmas
         }
     } // namespace
 
-    // Where one launch is the faster path (us per solve_device, iteration kernels -> one launch). Inverses,
-    // vectors and coarse lists in shared memory: always (8^3 FP64 1,240 -> 640, 20^3 FP16 1,870 -> 910,
-    // 33^3 FP16 3,120 -> 1,830, 200 x 100 plane FP16 3,800 -> 1,830). Inverses through the ring: while
-    // few batches pass per apply and a CTA has at most some 14 banks of 96 rows (23 of 64, 35 of 32):
-    // 37^3 FP32 3,850 -> 2,690, 33^3 FP64 3,730 -> 2,640, 400 x 200 plane FP64 5,960 -> 4,700, 52^3 scalar
-    // FP64 5,040 -> 4,200. Beyond, both are alike and then the kernels faster: 42^3 FP16 4,250 -> 4,150,
-    // 42^3 FP32 (8 batches) 4,700 -> 5,300, 45^3 FP16 4,980 -> 5,700, 500 x 250 plane FP64 (13 batches)
-    // 7,100 -> 9,100, 56^3 scalar FP64 5,270 -> 5,270.
+    // Where one launch is the faster path: up to persist_max_banks, with inverses, vectors and coarse lists in
+    // shared memory, or the inverses through the ring in at most 7 batches per apply. us per solve_device,
+    // iteration kernels -> one launch: 8^3 FP64 1,210 -> 650, 20^3 binary16 1,870 -> 940, 31^3 FP64 2,950 ->
+    // 2,710, 37^3 FP32 3,240 -> 2,820, 300^2 plane FP64 3,680 -> 3,240.
     PersistPlan persist_plan(const MasView &mas)
     {
         return dispatch_variant(mas.bd, mas.storage, [&]<int BD, class Store>() { return plan_variant<BD, Store>(mas); });
