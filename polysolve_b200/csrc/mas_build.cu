@@ -657,7 +657,9 @@ namespace pmas
 
         int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
-        // A copy in stream order, finished on return.
+        // A copy in stream order, finished on return. The buffers come from a stream-ordered pool
+        // (AllocScope) and s does not follow the legacy stream, so a plain cudaMemcpy would be ordered neither
+        // after the allocation nor before the kernels that read the copy.
         void copy_now(void *dst, const void *src, size_t bytes, cudaMemcpyKind kind, cudaStream_t s)
         {
             cuda_check(cudaMemcpyAsync(dst, src, bytes, kind, s), "copy");
@@ -1221,13 +1223,10 @@ namespace pmas
             M.n_coarse_active = (int)active.size();
             M.coarse_active.alloc(active.empty() ? 1 : active.size(), "MAS coarse_space active");
             if (!active.empty())
-                cuda_check(cudaMemcpy(M.coarse_active.get(), active.data(), active.size() * sizeof(int),
-                                      cudaMemcpyHostToDevice),
-                           "active");
+                copy_now(M.coarse_active.get(), active.data(), active.size() * sizeof(int), cudaMemcpyHostToDevice, s);
             M.parent.alloc(cn > 0 ? cn : 1, "MAS coarse_space parents");
             if (cn > 0)
-                cuda_check(cudaMemcpy(M.parent.get(), parent.data(), (size_t)cn * sizeof(int), cudaMemcpyHostToDevice),
-                           "parents");
+                copy_now(M.parent.get(), parent.data(), (size_t)cn * sizeof(int), cudaMemcpyHostToDevice, s);
             M.ticket.alloc(1, "MAS coarse_space ticket");
             cuda_check(cudaMemsetAsync(M.ticket.get(), 0, sizeof(unsigned), s), "memset");
             // Children lists (local ids) of the real nodes of levels 1..level_num-1.
@@ -1257,12 +1256,10 @@ namespace pmas
                 M.kid_ptr_all.alloc(ptr_all.empty() ? 1 : ptr_all.size(), "MAS coarse_space children");
                 M.kids.alloc(kid.empty() ? 1 : kid.size(), "MAS coarse_space children");
                 if (!ptr_all.empty())
-                    cuda_check(cudaMemcpy(M.kid_ptr_all.get(), ptr_all.data(), ptr_all.size() * sizeof(int),
-                                          cudaMemcpyHostToDevice),
-                               "children");
+                    copy_now(M.kid_ptr_all.get(), ptr_all.data(), ptr_all.size() * sizeof(int), cudaMemcpyHostToDevice,
+                             s);
                 if (!kid.empty())
-                    cuda_check(cudaMemcpy(M.kids.get(), kid.data(), kid.size() * sizeof(int), cudaMemcpyHostToDevice),
-                               "children");
+                    copy_now(M.kids.get(), kid.data(), kid.size() * sizeof(int), cudaMemcpyHostToDevice, s);
             }
         }
 
