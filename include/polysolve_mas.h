@@ -196,7 +196,12 @@ int mas_set_stream(mas_solver *h, void *stream);
  * allocations). d_x, d_y: device vectors of length len = nodes * block_dim in the solver's padded
  * block order (see mas_get_sizes); d_dot: one device double. The three buffers must not overlap
  * (MAS_ERR_INVALID otherwise). Runs on `stream` (a cudaStream_t, NULL = the handle's stream)
- * without synchronizing. The reduction scratch is a static device array of 256 KB + 8 B (held by
+ * without synchronizing; d_x, d_y and d_dot must stay until it has run. The handle's own memory does: after
+ * such a call on a stream other than the handle's, the next factorization of another pattern and
+ * mas_destroy wait for the device first, and each of them does after a call inside a stream capture
+ * (whose graph must not be launched once the pattern has changed or the handle is gone; a
+ * factorization that keeps the pattern overwrites the values in place, so order it after the
+ * products that want the old ones). The reduction scratch is a static device array of 256 KB + 8 B (held by
  * every GPU where the library's module is loaded, until exit), which limits the matrix to 262,144
  * banks (8,388,608 block rows); larger matrices get MAS_ERR_INVALID. All calls share that scratch:
  * calls that overlap on the GPU race. The first call on a device (and the first after a

@@ -447,12 +447,27 @@ struct mas_solver
     bool last_multi = false; // the last solve was a several-right-hand-side solve
     PcgState *h_st = nullptr; // pinned, 2 slots
 
+    // Products of mas_spmv_dot_noalloc that may still read the matrix on a stream the handle does not wait
+    // for: one since the last release, or one captured into a graph that may run at any time.
+    std::atomic<bool> product_outside{false}, product_captured{false};
+
+    // Before the matrix's buffers are released: they return to a stream-ordered pool (AllocScope), or by a
+    // cudaFree that does not wait for memory of such a pool, so products outside the handle's stream are
+    // waited for here.
+    void wait_products()
+    {
+        if (product_outside.exchange(false) || product_captured.load())
+            cuda_check(cudaDeviceSynchronize(), "products in flight");
+    }
+
     ~mas_solver()
     {
         if (stream)
         {
             cudaSetDevice(device);
             cudaStreamSynchronize(stream);
+            if (product_outside.load() || product_captured.load())
+                cudaDeviceSynchronize();
         }
         for (cudaEvent_t e : ev_pool)
             cudaEventDestroy(e);
@@ -830,6 +845,7 @@ struct mas_solver
                 d_inner.alloc(nnz_ > 0 ? nnz_ : 1, "MAS permuted_bsr input_csc");
                 upload_pageable(d_outer.get(), outer, sizeof(int) * (size_t)(n_ + 1));
                 upload_pageable(d_inner.get(), inner, sizeof(int) * (size_t)nnz_);
+                wait_products();
                 A.slice.reset();
                 A.cols.reset();
                 A.vals.reset();
@@ -2913,7 +2929,14 @@ extern "C" int mas_spmv_dot_noalloc(mas_solver *h, const double *d_x, double *d_
         if ((x0 < y0 + bytes && y0 < x0 + bytes) || inside(dot, x0, bytes) || inside(dot, y0, bytes))
             throw Error(ERR_INVALID, "[MAS] spmv_dot_noalloc: d_x, d_y and d_dot must not overlap.");
         cuda_check(cudaSetDevice(h->device), "set device");
-        launch_spmv_dot_noalloc(h->A.view(), d_x, d_y, d_dot, stream ? static_cast<cudaStream_t>(stream) : h->stream);
+        const cudaStream_t on = stream ? static_cast<cudaStream_t>(stream) : h->stream;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        cuda_check(cudaStreamIsCapturing(on, &capture), "capture status");
+        if (capture != cudaStreamCaptureStatusNone)
+            h->product_captured.store(true);
+        else if (on != h->stream)
+            h->product_outside.store(true);
+        launch_spmv_dot_noalloc(h->A.view(), d_x, d_y, d_dot, on);
     });
 }
 
