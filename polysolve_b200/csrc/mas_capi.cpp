@@ -405,10 +405,10 @@ struct mas_solver
     DevBuf<PcgState> st;
     DevBuf<double> partials;
     int red_capacity = 0;
-    // The one-launch solve of small systems (mas_persist.cu): its dots and barrier counter, allocated
-    // with the other vectors when the system is small enough.
+    // The one-launch solve of small systems (mas_persist.cu): its dots and gathered vectors, allocated
+    // with the others when the system is small enough. Its barrier counter is the word behind the
+    // state (st has two records), so that one copy brings both to h_st.
     DevBuf<double> persist_dots, persist_gather;
-    DevBuf<unsigned> persist_bar;
     bool persist_ready = false;
     double l2_bytes = 0.0;
     bool in_batch = false; // solving as one of several systems of mas_solve_batch
@@ -914,7 +914,7 @@ struct mas_solver
         z.alloc(len, "device_buffers z");
         Ap.alloc(len, "device_buffers Ap");
         io.alloc((size_t)n_ > len ? (size_t)n_ : len, "device_buffers io");
-        st.alloc(1, "device_buffers scalars");
+        st.alloc(2, "device_buffers scalars");
         red_capacity = std::max({(banks + 7) / 8, mas.total_coarse, device_sm_count() * 8}) + 160;
         partials.alloc((size_t)red_capacity * 9, "device_buffers reduction");
         persist_ready = banks <= PERSIST_MAX_BANKS && prepare_persistent(bd_, p.storage);
@@ -923,7 +923,6 @@ struct mas_solver
             persist_dots.alloc(3 * (size_t)((banks + 7) & ~7) + 3 * (size_t)device_sm_count() * 16 + 2,
                                "device_buffers reduction");
             persist_gather.alloc(persist_gather_size(mas.view()), "device_buffers p");
-            persist_bar.alloc(1, "device_buffers reduction");
             cuda_check(cudaMemsetAsync(persist_dots.get(), 0, persist_dots.bytes(), stream), "memset");
         }
         cuda_check(cudaMemsetAsync(x.get(), 0, x.bytes(), stream), "memset");
@@ -1096,19 +1095,26 @@ struct mas_solver
     }
 
     // The whole solve in one launch (a long one in slices, so that no launch runs for seconds); the
-    // caller reads h_st[0] after its synchronisation.
+    // caller reads h_st[0] after its synchronisation; a wait that ran out anywhere makes it ERR_TIMEOUT.
     void pcg_persistent(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, const PersistPlan &pl)
     {
         constexpr int SLICE = 2048;
         PcgState *S = st.get();
+        unsigned *bar = reinterpret_cast<unsigned *>(S + 1);
         for (int k0 = 0; k0 == 0 || (k0 < p.max_iter && !h_st[0].done); k0 += SLICE)
         {
             run("pcg_persistent", 1, [&] {
                 launch_pcg_persistent(Av, mv, cfg, pl, S, x.get(), r.get(), persist_gather.get(), b.get(),
-                                      persist_dots.get(), persist_bar.get(), k0 == 0 ? 1 : 0, SLICE, p.true_residual_period, stream);
+                                      persist_dots.get(), bar, k0 == 0 ? 1 : 0, SLICE, p.true_residual_period, stream);
             });
-            cuda_check(cudaMemcpyAsync(&h_st[0], S, sizeof(PcgState), cudaMemcpyDeviceToHost, stream), "state");
+            cuda_check(cudaMemcpyAsync(&h_st[0], S, sizeof(PcgState) + sizeof(unsigned), cudaMemcpyDeviceToHost, stream),
+                       "state");
             cuda_check(cudaStreamSynchronize(stream), "pcg");
+            if (*reinterpret_cast<const unsigned *>(&h_st[1]) & PERSIST_ABORT)
+            {
+                h_st[0].error = ERR_TIMEOUT;
+                return;
+            }
         }
     }
 

@@ -299,7 +299,8 @@ namespace pmas
         unsigned int counter[8];
     };
 
-    // Default iteration limit of a bounded device-side wait (an mbarrier wait of a bulk copy).
+    // Default iteration limit of a bounded device-side wait (an mbarrier wait of a bulk copy, a grid barrier of
+    // the one-launch solve).
     constexpr long long MBAR_SPIN_LIMIT_DEFAULT = 1LL << 20;
 
     struct PcgConfig
@@ -589,9 +590,11 @@ namespace pmas
     // mas_persist.cu: a whole single-right-hand-side solve in one launch, for small systems. The plan
     // says whether the system fits (ok) and the launch shape; dots: persist_dots_size doubles, zeroed
     // once after a factorization; gather: persist_gather_size doubles (p and x as the SpMV gathers
-    // them; kept between the launches of one solve); bar: one counter. first: start the solve, otherwise go on where the
+    // them; kept between the launches of one solve); bar: one counter, in which a wait that ran out leaves
+    // PERSIST_ABORT (the solve is incomplete then, whatever *st says). first: start the solve, otherwise go on where the
     // launch before stopped; at most `iters` iterations per launch.
     constexpr int PERSIST_MAX_BANKS = 5200; // no plan beyond
+    constexpr unsigned PERSIST_ABORT = 0x80000000u;
     struct PersistPlan
     {
         bool ok = false;

@@ -35,9 +35,6 @@ namespace pmas
     {
         constexpr int PS_THREADS = 384;
         constexpr int PS_WARPS = PS_THREADS / 32;
-        constexpr unsigned PS_ABORT = 0x80000000u;
-        // Polls of a grid barrier before the solve gives up (some seconds).
-        constexpr int PS_SPIN_LIMIT = 1 << 22;
 
         // Per-warp scratch of the apply: the binary16 hi / lo input and 32 result rows, or the FP32 input.
         template <int BD, class Store>
@@ -111,8 +108,10 @@ namespace pmas
             asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
         }
 
-        // Grid barrier: arrive, then wait. Monotonic arrival count (no reset inside a launch); the top
-        // bit tells every CTA that one gave up. A wait that runs out sets it too.
+        // Grid barrier: arrive, then wait, for at most `limit` polls (some 0.5 us each). Monotonic arrival
+        // count (no reset inside a launch); its top bit (PERSIST_ABORT) tells every CTA that one gave up. A
+        // wait that runs out sets it too, and it is the only record of that: the others may be past the
+        // barrier by then, and through with the solve.
         __device__ __forceinline__ void ps_arrive(unsigned *bar)
         {
             __syncthreads();
@@ -120,7 +119,7 @@ namespace pmas
                 red_release_gpu(bar, 1u);
         }
 
-        __device__ __forceinline__ bool ps_wait(unsigned *bar, unsigned &target)
+        __device__ __forceinline__ bool ps_wait(unsigned *bar, unsigned &target, long long limit)
         {
             target += gridDim.x;
             bool gave_up = false;
@@ -128,19 +127,19 @@ namespace pmas
             {
                 unsigned v = 0;
 #pragma unroll 1
-                for (int i = 0; i < PS_SPIN_LIMIT && v < target; ++i)
+                for (long long i = 0; i < limit && v < target; ++i)
                     v = ld_acquire_gpu(bar); // the abort bit ends the wait too
-                gave_up = v < target || (v & PS_ABORT);
+                gave_up = v < target || (v & PERSIST_ABORT);
                 if (gave_up)
-                    atomicOr(bar, PS_ABORT);
+                    atomicOr(bar, PERSIST_ABORT);
             }
             return !__syncthreads_or(gave_up);
         }
 
-        __device__ __forceinline__ bool ps_barrier(unsigned *bar, unsigned &target)
+        __device__ __forceinline__ bool ps_barrier(unsigned *bar, unsigned &target, long long limit)
         {
             ps_arrive(bar);
-            return ps_wait(bar, target);
+            return ps_wait(bar, target, limit);
         }
 
         // Global dots (written before the last grid barrier) into shared memory, 16 bytes per thread and
@@ -595,7 +594,7 @@ namespace pmas
             // Without its inverses and rows the CTA must not go on: it tells the others and leaves.
             bool ok = __syncthreads_and(mbar_wait_bounded(&sh.bar, 0u, nullptr, a.cfg.wait_limit)) != 0;
             if (!ok && tid == 0)
-                atomicOr(a.bar, PS_ABORT);
+                atomicOr(a.bar, PERSIST_ABORT);
             unsigned target = 0;
             int batch = 0; // batches multiplied in this launch
             bool gave_up = false; // a wait for a batch ran out
@@ -614,7 +613,7 @@ namespace pmas
             }
             // x is where the first residual gathers it once every CTA is past this barrier (which also
             // orders the table above).
-            ok = ps_barrier(a.bar, target) && ok;
+            ok = ps_barrier(a.bar, target, a.cfg.wait_limit) && ok;
 
 #pragma unroll 1
             for (int n = a.first ? -1 : 0; ok; ++n)
@@ -670,7 +669,7 @@ namespace pmas
                     }
                     if (residual)
                         break;
-                    if (!(ok = ps_barrier(a.bar, target)))
+                    if (!(ok = ps_barrier(a.bar, target, a.cfg.wait_limit)))
                         break;
                     stage_dots<0>(dot_pap, bank_pad, 0, bank_pad, staged);
                     __syncthreads();
@@ -714,7 +713,7 @@ namespace pmas
                     }
                     if (!residual)
                         break;
-                    if (!(ok = ps_barrier(a.bar, target)))
+                    if (!(ok = ps_barrier(a.bar, target, a.cfg.wait_limit)))
                         break;
                 }
                 if (!ok)
@@ -742,7 +741,7 @@ namespace pmas
                 {
                     if (part == 1)
                     {
-                        if (!(ok = ps_wait(a.bar, target)) || nb == ni)
+                        if (!(ok = ps_wait(a.bar, target, a.cfg.wait_limit)) || nb == ni)
                             break;
                         // Coarse levels above the first, four nodes per warp: eight lanes per node, four of its
                         // children each, added in the order of the warp sums of k_coarse_levels (children 16
@@ -827,7 +826,7 @@ namespace pmas
                 if (!ok)
                     break;
                 if (__syncthreads_or(gave_up) && tid == 0)
-                    atomicOr(a.bar, PS_ABORT); // barrier C below tells every CTA
+                    atomicOr(a.bar, PERSIST_ABORT); // barrier C below tells every CTA
                 // ---- r.z per team: its coupled banks in order, then the warp sum. A team has at most one item
                 // beyond them (an isolated bank or a coarse matrix): its dot on its own, by item.
 #pragma unroll 1
@@ -861,7 +860,7 @@ namespace pmas
                             dot_rz[team_pad + extra] = beyond;
                     }
                 }
-                if (!(ok = ps_barrier(a.bar, target)))
+                if (!(ok = ps_barrier(a.bar, target, a.cfg.wait_limit)))
                     break;
                 // ---- Totals and the scalar step, in every CTA. The coarse corrections of the warp's first
                 // rows of p are on their way meanwhile.
@@ -986,7 +985,7 @@ namespace pmas
                 }
                 if (!pdo || n + 1 == a.iters)
                     break;
-                ok = ps_barrier(a.bar, target);
+                ok = ps_barrier(a.bar, target, a.cfg.wait_limit);
             }
 
             // ---- Out: x, r, the state; no copy may be in flight when the CTA leaves.
@@ -1011,15 +1010,8 @@ namespace pmas
                     for (long long i = 0; i < MBAR_SPIN_LIMIT; ++i)
                         if (mbar_try_wait(&sh.ring_bar[g % buffers], (uint32_t)(g / buffers) & 1u))
                             break;
-                if (!ok)
-                {
-                    sh.st.error = ERR_TIMEOUT;
-                    sh.st.done = 1;
-                }
                 if (blockIdx.x == 0)
                     *a.st = sh.st;
-                else if (!ok)
-                    atomicExch(&a.st->error, ERR_TIMEOUT);
             }
         }
 
