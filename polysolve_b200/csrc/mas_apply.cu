@@ -94,7 +94,7 @@ namespace pmas
             // for the predecessor (launched chained in a PCG iteration), or at the first coarse matrix.
             if (!early)
                 pdl_wait();
-            if (MODE != 0 && st->done)
+            if (MODE != 0 && __ldcg(&st->done))
             {
                 if (lane == 0)
                     mbar_drain(bar, pending, {0u, 0u});
@@ -303,7 +303,7 @@ namespace pmas
             // for the predecessor (launched chained in a PCG iteration), or at the first coarse matrix.
             if (!early)
                 pdl_wait();
-            if (MODE != 0 && st->done)
+            if (MODE != 0 && __ldcg(&st->done))
             {
                 if (loader)
                     mbar_drain(bar, pending, {0u, 0u});
@@ -416,8 +416,8 @@ namespace pmas
 
         // early: the predecessor in the stream is k_coarse_levels, which lets this kernel start once its
         // own predecessor (the producer of r) has completed. The level-0 matrices then go ahead while the
-        // coarse levels are summed, and pdl_wait() comes before the first coarse input. r and rc are read
-        // past L1 (__ldcg): r's producer was not waited for by this grid itself.
+        // coarse levels are summed, and pdl_wait() comes before the first coarse input. r, rc and st->done are
+        // read past L1 (__ldcg): their producers were not waited for by this grid itself.
         // (One after the other, an iteration took 53.8 us at 44^3 in binary16, 49.7 us at 70^3 scalar FP64
         // and 180.5 us at 80^3, now 47.5, 44.0 and 172.7 us.)
         template <int BD, class Store, int MODE>

@@ -1,7 +1,11 @@
-"""Order of the factorization's copies. Its buffers come from a stream-ordered pool and are used on the
+"""Orders of memory accesses that no run shows to be wrong reliably, so the sources are read instead.
+
+The factorization's copies: its buffers come from a stream-ordered pool and are used on the
 handle's non-blocking stream, which does not follow the legacy stream: a synchronous copy or set
-there would run beside the allocation it writes to and the kernels that read it. Such a race shows on
-no run that can be relied on, so the sources are read instead."""
+there would run beside the allocation it writes to and the kernels that read it.
+
+The MAS apply that starts beside the coarse sums: it has not waited for the kernel before them itself, so
+what that kernel and earlier ones wrote is read past L1."""
 
 from __future__ import annotations
 
@@ -30,3 +34,14 @@ def test_factorization_copies_follow_the_stream(name):
     # Every launch names its stream (the fourth launch argument).
     for launch in re.findall(r"<<<(.*?)>>>", text, flags=re.S):
         assert re.search(r",\s*(s|stream)\s*$", launch), launch
+
+
+@pytest.mark.parametrize("form", ["mas_apply_warps", "mas_apply_rows"])
+def test_early_apply_reads_past_l1(form):
+    text = _code((CSRC / "mas_apply.cu").read_text())
+    start = text.index(f"bool {form}(")
+    body = text[start:text.index("return true;", start)]
+    assert "__ldcg(&st->done)" in body
+    assert re.findall(r"(?<!__ldcg\(&)st->done", body) == []
+    assert "__ldcg(in + " in body
+    assert re.findall(r"\bin\[", body) == []
