@@ -299,9 +299,11 @@ namespace
 
 namespace
 {
-    // The memory pool a handle factorizes with (AllocScope): freed temporaries of up to KEEP bytes stay in
-    // it for the next factorization, the rest and everything at the handle's end goes back to the device.
-    // Declared before the handle's buffers, so it is destroyed after them.
+    // The memory pool a handle factorizes with (AllocScope). It holds on to KEEP bytes, the handle's live
+    // buffers among them: freed temporaries of smaller systems stay in it for the next factorization, those
+    // that would bring it above go back to the device at the next wait for the stream, and so does
+    // everything at the handle's end or when an allocation fails anywhere (device_alloc). Declared before
+    // the handle's buffers, so it is destroyed after them.
     struct AllocPool
     {
         static constexpr uint64_t KEEP = 256ull << 20;
@@ -322,12 +324,15 @@ namespace
             }
             uint64_t keep = KEEP;
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            register_pool(pool, device);
             return pool;
         }
         ~AllocPool()
         {
-            if (pool)
-                cudaMemPoolDestroy(pool);
+            if (!pool)
+                return;
+            unregister_pool(pool);
+            cudaMemPoolDestroy(pool);
         }
     };
 } // namespace

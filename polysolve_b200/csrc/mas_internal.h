@@ -64,6 +64,10 @@ namespace pmas
         AllocScope &operator=(const AllocScope &) = delete;
     };
 
+    // The pools whose unused memory a failing allocation gives back (registered while they live).
+    void register_pool(cudaMemPool_t pool, int device);
+    void unregister_pool(cudaMemPool_t pool);
+
     // throws Error(ERR_OOM) with MB figures; *pooled: the memory came from the thread's AllocScope
     void *device_alloc(size_t bytes, const char *ctx, bool *pooled);
     void device_free(void *p, bool pooled);

@@ -15,6 +15,7 @@
 #include <mutex>
 #include <string>
 #include <unordered_map>
+#include <vector>
 
 #include "mas_common.cuh"
 
@@ -47,7 +48,37 @@ namespace pmas
         t_alloc_stream = saved_stream;
     }
 
-    // Allocation with the reference's out-of-memory message (mas_utils/CudaUtils.cuh:68-79).
+    // Every live pool with its device: an allocation that fails gives back what they hold unused.
+    static std::mutex g_pools_mutex;
+    static std::vector<std::pair<cudaMemPool_t, int>> g_pools;
+
+    void register_pool(cudaMemPool_t pool, int device)
+    {
+        std::lock_guard<std::mutex> lock(g_pools_mutex);
+        g_pools.push_back({pool, device});
+    }
+
+    void unregister_pool(cudaMemPool_t pool)
+    {
+        std::lock_guard<std::mutex> lock(g_pools_mutex);
+        std::erase_if(g_pools, [&](const auto &e) { return e.first == pool; });
+    }
+
+    static void trim_pools()
+    {
+        int device = 0;
+        cudaGetDevice(&device);
+        if (t_alloc_pool)
+            cudaStreamSynchronize(t_alloc_stream); // this thread's own frees
+        std::lock_guard<std::mutex> lock(g_pools_mutex);
+        for (const auto &e : g_pools)
+            if (e.second == device)
+                cudaMemPoolTrimTo(e.first, 0);
+        cudaGetLastError();
+    }
+
+    // Allocation with the reference's out-of-memory message (mas_utils/CudaUtils.cuh:68-79). Where it
+    // fails, the unused memory of all pools of the device goes back first and it is tried once more.
     void *device_alloc(size_t bytes, const char *ctx, bool *pooled)
     {
         void *p = nullptr;
@@ -64,10 +95,17 @@ namespace pmas
                 break;
             }
         }
-        if (!injected)
-            e = *pooled ? cudaMallocFromPoolAsync(&p, bytes, t_alloc_pool, t_alloc_stream) : cudaMalloc(&p, bytes);
-        if (e == cudaSuccess)
-            return p;
+        for (int attempt = 0; attempt < 2; ++attempt)
+        {
+            if (!injected)
+                e = *pooled ? cudaMallocFromPoolAsync(&p, bytes, t_alloc_pool, t_alloc_stream) : cudaMalloc(&p, bytes);
+            if (e == cudaSuccess)
+                return p;
+            if (e != cudaErrorMemoryAllocation || attempt > 0)
+                break;
+            cudaGetLastError();
+            trim_pools();
+        }
         if (e != cudaErrorMemoryAllocation)
             cuda_check(e, ctx);
         cudaGetLastError();
