@@ -277,9 +277,30 @@ namespace
 
     std::string g_create_error;
 
+    // The solves in progress on each device, over all handles and threads. A cooperative launch keeps its
+    // SMs to itself for the whole solve, so one that leaves the others few is for a solve that found none
+    // in progress; beside another solve the iteration kernels (the same bits) overlap. us per solve of 20^3
+    // in binary16 from 4 and 8 threads, one launch whenever no other was cooperative / this rule: 813 / 440 and
+    // 696 / 393; a 44^3 solve beside such solves in a loop: 30 / 4.5 ms, beside 14^3 ones 7.8 / 4.2 ms. Up to
+    // a quarter of the SMs it costs the others nothing (8^3: 4.2 / 4.0 ms, itself 0.70 / 1.37 ms).
+    struct RunningSolve
+    {
+        static std::atomic<int> running[64];
+        int device;
+        bool alone;
+        explicit RunningSolve(int dev) : device(dev), alone(dev >= 0 && dev < 64 && running[dev].fetch_add(1) == 0) {}
+        RunningSolve(const RunningSolve &) = delete;
+        RunningSolve &operator=(const RunningSolve &) = delete;
+        ~RunningSolve()
+        {
+            if (device >= 0 && device < 64)
+                running[device].fetch_sub(1);
+        }
+    };
+    std::atomic<int> RunningSolve::running[64];
+
     // One cooperative solve at a time on each device: its CTAs wait for one another, so two of them
-    // must not hold parts of the device each. A thread that finds the device taken uses the iteration
-    // kernels (the same bits), as it would overlap with the other solve's kernels anyway.
+    // must not hold parts of the device each.
     struct CooperativeTurn
     {
         static std::atomic<bool> taken[64];
@@ -417,6 +438,7 @@ struct mas_solver
     bool persist_ready = false;
     double l2_bytes = 0.0;
     bool in_batch = false; // solving as one of several systems of mas_solve_batch
+    bool alone = false;    // the solve began with no other in progress on the device
 
     // Several right-hand sides at once: groups of RHS_GROUP interleaved vectors, one PcgState
     // per right-hand side plus the group record, their own graphs.
@@ -1088,12 +1110,15 @@ struct mas_solver
 
     // The shape of the one-launch solve, or one that is not ok: the iteration kernels run instead for
     // larger systems, Polak-Ribiere (its r.z_old dots), per-kernel profiling, host-launched iterations
-    // (cuda_graphs off) and in batches, where other systems' kernels fill the device.
+    // (cuda_graphs off), and in batches and (but for the smallest) beside other solves, whose kernels fill
+    // the device.
     PersistPlan persistent_plan(const MasView &mv, const PcgConfig &cfg) const
     {
         PersistPlan pl;
         if (persist_ready && p.graphs && !p.profile && !in_batch && !cfg.polak_ribiere && p.max_iter >= 1)
             pl = persist_plan(mv);
+        if (pl.ok && !alone && pl.grid > device_sm_count() / 4)
+            pl.ok = false;
         if (pl.ok && persist_dots_size(mv, pl) > persist_dots.n)
             pl.ok = false;
         return pl;
@@ -1857,6 +1882,7 @@ struct mas_solver
             in_multi = false;
             return;
         }
+        const RunningSolve turn(device);
         const int W = group_width(nrhs);
         alloc_multi(W);
         for (auto &ks : kstats)
@@ -1905,6 +1931,8 @@ struct mas_solver
         last_multi = false;
         if (!hb || !hx)
             throw Error(ERR_INVALID, "[MAS] solve: null vector.");
+        const RunningSolve turn(device);
+        alone = turn.alone;
         cuda_check(cudaMemcpyAsync(io.get(), hb, sizeof(double) * n, cudaMemcpyHostToDevice, stream), "upload b");
         const size_t blen = (size_t)banks * 32 * bd;
         run("permute_in", 2, [&] { launch_permute_in(n, bd, V, d_padded.get(), io.get(), b.get(), blen, stream); });
@@ -2075,6 +2103,8 @@ struct mas_solver
         cuda_check(cudaSetDevice(device), "set device");
         require_factorized(len);
         last_multi = false;
+        const RunningSolve turn(device);
+        alone = turn.alone;
         load_rhs_device(d_b, learned_active() ? nullptr : d_x);
         if (learned_active())
             warm_start_guess();
@@ -2546,6 +2576,7 @@ namespace
                 return false;
         }
         const int dev = handles[0]->device;
+        const RunningSolve turn(dev);
         cuda_check(cudaSetDevice(dev), "set device");
         set_apply_items_per_warp(p0.apply_ipw); // the apply grids below are the handles' own
         // Input steps; systems whose input is rejected keep their error and leave the batch.
