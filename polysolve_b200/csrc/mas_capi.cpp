@@ -277,10 +277,10 @@ namespace
 
     std::string g_create_error;
 
-    // The solves in progress on each device, over all handles and threads. A cooperative launch keeps its
-    // SMs to itself for the whole solve, so one that leaves the others few is for a solve that found none
+    // The solves in progress on each device, over all handles and threads. A one-launch solve keeps its
+    // SMs to itself all the time, so one that leaves the others few is for a solve that found none
     // in progress; beside another solve the iteration kernels (the same bits) overlap. us per solve of 20^3
-    // in binary16 from 4 and 8 threads, one launch whenever no other was cooperative / this rule: 813 / 440 and
+    // in binary16 from 4 and 8 threads, one launch whenever no other had one / this rule: 813 / 440 and
     // 696 / 393; a 44^3 solve beside such solves in a loop: 30 / 4.5 ms, beside 14^3 ones 7.8 / 4.2 ms. Up to
     // a quarter of the SMs it costs the others nothing (8^3: 4.2 / 4.0 ms, itself 0.70 / 1.37 ms).
     struct RunningSolve
@@ -299,23 +299,23 @@ namespace
     };
     std::atomic<int> RunningSolve::running[64];
 
-    // One cooperative solve at a time on each device: its CTAs wait for one another, so two of them
-    // must not hold parts of the device each.
-    struct CooperativeTurn
+    // One one-launch solve at a time on each device: its CTAs wait for one another, so two of them
+    // must not hold parts of the device each (both would be called off).
+    struct OneLaunchTurn
     {
         static std::atomic<bool> taken[64];
         int device;
         bool mine;
-        explicit CooperativeTurn(int dev) : device(dev), mine(dev >= 0 && dev < 64 && !taken[dev].exchange(true)) {}
-        CooperativeTurn(const CooperativeTurn &) = delete;
-        CooperativeTurn &operator=(const CooperativeTurn &) = delete;
-        ~CooperativeTurn()
+        explicit OneLaunchTurn(int dev) : device(dev), mine(dev >= 0 && dev < 64 && !taken[dev].exchange(true)) {}
+        OneLaunchTurn(const OneLaunchTurn &) = delete;
+        OneLaunchTurn &operator=(const OneLaunchTurn &) = delete;
+        ~OneLaunchTurn()
         {
             if (mine)
                 taken[device].store(false);
         }
     };
-    std::atomic<bool> CooperativeTurn::taken[64];
+    std::atomic<bool> OneLaunchTurn::taken[64];
 } // namespace
 
 namespace
@@ -1126,26 +1126,41 @@ struct mas_solver
 
     // The whole solve in one launch (a long one in slices, so that no launch runs for seconds); the
     // caller reads h_st[0] after its synchronisation; a wait that ran out anywhere makes it ERR_TIMEOUT.
-    void pcg_persistent(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, const PersistPlan &pl)
+    // Returns false where a launch did not get its SMs in time: the iteration kernels go on from iteration
+    // `done` then, whose p is in the SpMV's gathering order.
+    bool pcg_persistent(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, const PersistPlan &pl, int &done)
     {
         constexpr int SLICE = 2048;
         PcgState *S = st.get();
         unsigned *bar = reinterpret_cast<unsigned *>(S + 1);
-        for (int k0 = 0; k0 == 0 || (k0 < p.max_iter && !h_st[0].done); k0 += SLICE)
+        for (done = 0; done == 0 || (done < p.max_iter && !h_st[0].done); done += SLICE)
         {
             run("pcg_persistent", 1, [&] {
                 launch_pcg_persistent(Av, mv, cfg, pl, S, x.get(), r.get(), persist_gather.get(), b.get(),
-                                      persist_dots.get(), bar, k0 == 0 ? 1 : 0, SLICE, p.true_residual_period, stream);
+                                      persist_dots.get(), bar, done == 0 ? 1 : 0, SLICE, p.true_residual_period, stream);
             });
             cuda_check(cudaMemcpyAsync(&h_st[0], S, sizeof(PcgState) + sizeof(unsigned), cudaMemcpyDeviceToHost, stream),
                        "state");
             cuda_check(cudaStreamSynchronize(stream), "pcg");
-            if (*reinterpret_cast<const unsigned *>(&h_st[1]) & PERSIST_ABORT)
+            const unsigned end = *reinterpret_cast<const unsigned *>(&h_st[1]);
+            if (end & PERSIST_LATE)
+                return false;
+            if (end & PERSIST_ABORT)
             {
                 h_st[0].error = ERR_TIMEOUT;
-                return;
+                return true;
             }
         }
+        return true;
+    }
+
+    // p as the iteration kernels hold it, from the one-launch solve's (persist_gather_size).
+    void gathered_p()
+    {
+        const size_t width = sizeof(double) * bd, pitch = bd == 3 ? 4 * sizeof(double) : width;
+        cuda_check(cudaMemcpy2DAsync(pv.get(), width, persist_gather.get(), pitch, width, (size_t)banks * 32,
+                                     cudaMemcpyDeviceToDevice, stream),
+                   "p");
     }
 
     // pcg_solve (MASSolver.cu:469-595) on device-resident b_ / x_ (padded order).
@@ -1167,16 +1182,18 @@ struct mas_solver
         set_chained_launch(p.chained);
         set_spmv_unroll(p.spmv_unroll);
         set_apply_items_per_warp(p.apply_ipw);
-        PersistPlan pl = persistent_plan(mv, cfg);
-        if (pl.ok)
+        const PersistPlan pl = persistent_plan(mv, cfg);
+        bool one_launch = pl.ok;
+        int done = 0; // iterations of a one-launch solve that the iteration kernels go on with
+        if (one_launch)
         {
-            CooperativeTurn turn(device);
-            pl.ok = turn.mine;
-            if (pl.ok)
-                pcg_persistent(Av, mv, cfg, pl); // returns when the launch has finished
+            OneLaunchTurn turn(device);
+            one_launch = turn.mine && pcg_persistent(Av, mv, cfg, pl, done); // returns when the launch has finished
         }
-        if (!pl.ok)
+        if (!one_launch && done == 0)
             pcg_start(Av, mv, cfg);
+        else if (!one_launch)
+            gathered_p();
         rz0 = h_st[0].rz0;
         rr0 = h_st[0].rr0;
         if (h_st[0].error == ERR_TIMEOUT)
@@ -1192,14 +1209,14 @@ struct mas_solver
             throw Error(ERR_NONFINITE, "[MAS] Invalid initial residual.");
         }
         status = MAS_STATUS_RUNNING;
-        if (pl.ok)
+        if (one_launch)
         {
             cuda_check(cudaEventRecord(e1, stream), "event");
             cuda_check(cudaEventSynchronize(e1), "pcg");
             launched_iterations = h_st[0].iter;
         }
         else
-            launched_iterations = pcg_iterate(Av, mv, cfg, e1);
+            launched_iterations = pcg_iterate(Av, mv, cfg, done + 1, e1);
         collect_profile();
         ev_origin = nullptr;
         float ms = 0.f;
@@ -1232,15 +1249,15 @@ struct mas_solver
         cuda_check(cudaStreamSynchronize(stream), "pcg init");
     }
 
-    // The iterations of a solve by the iteration kernels, in chunks of poll_period, until a chunk's
-    // state says done; records e1 after the last one. Returns the iterations launched; h_st[0] holds
-    // the final state.
-    int pcg_iterate(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, cudaEvent_t e1)
+    // The iterations of a solve by the iteration kernels from `first` on, in chunks of poll_period, until a
+    // chunk's state says done; records e1 after the last one. Returns the last iteration launched; h_st[0]
+    // holds the final state. (The graphs are made for chunks that start at iteration 1.)
+    int pcg_iterate(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, int first, cudaEvent_t e1)
     {
         PcgState *S = st.get();
         const int P = p.true_residual_period;
         const int chunk = p.poll_period;
-        const bool graphs = p.graphs && !p.profile;
+        const bool graphs = p.graphs && !p.profile && first == 1;
         if (graphs)
             ensure_graph(Av, mv, cfg, P, chunk);
         int launched = 0;
@@ -1250,7 +1267,7 @@ struct mas_solver
         cuda_check(cudaEventCreateWithFlags(&chunk_ev[0], cudaEventDisableTiming), "event");
         cuda_check(cudaEventCreateWithFlags(&chunk_ev[1], cudaEventDisableTiming), "event");
         int slot_flip = 0;
-        for (int k0 = 1; k0 <= p.max_iter && !stop; k0 += chunk)
+        for (int k0 = first; k0 <= p.max_iter && !stop; k0 += chunk)
         {
             const int k1 = std::min(p.max_iter, k0 + chunk - 1);
             if (graphs)

@@ -595,10 +595,11 @@ namespace pmas
     // says whether the system fits (ok) and the launch shape; dots: persist_dots_size doubles, zeroed
     // once after a factorization; gather: persist_gather_size doubles (p and x as the SpMV gathers
     // them; kept between the launches of one solve); bar: one counter, in which a wait that ran out leaves
-    // PERSIST_ABORT (the solve is incomplete then, whatever *st says). first: start the solve, otherwise go on where the
+    // PERSIST_ABORT (the solve is incomplete then, whatever *st says); with PERSIST_LATE the launch did not
+    // get the SMs it needs in time and has changed neither x and r nor *st. first: start the solve, otherwise go on where the
     // launch before stopped; at most `iters` iterations per launch.
     constexpr int PERSIST_MAX_BANKS = 5200; // no plan beyond
-    constexpr unsigned PERSIST_ABORT = 0x80000000u;
+    constexpr unsigned PERSIST_ABORT = 0x80000000u, PERSIST_LATE = 0x40000000u;
     struct PersistPlan
     {
         bool ok = false;
@@ -606,7 +607,7 @@ namespace pmas
             staged = 0;
         size_t smem = 0;
     };
-    bool prepare_persistent(int bd, int storage); // false: no cooperative launch of this shape here
+    bool prepare_persistent(int bd, int storage); // false: no launch of this shape here
     PersistPlan persist_plan(const MasView &mas);
     size_t persist_dots_size(const MasView &mas, const PersistPlan &pl);
     size_t persist_gather_size(const MasView &mas);

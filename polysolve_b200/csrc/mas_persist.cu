@@ -94,6 +94,7 @@ namespace pmas
             uint64_t bar, ring_bar[2];
             int deep_top, deep_lo, deep_hi; // coarse levels above the first: highest level this CTA needs,
                                             // its range of level-1 nodes
+            int began; // every CTA had its SM in time
         };
 
         __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p)
@@ -134,6 +135,40 @@ namespace pmas
                     atomicOr(bar, PERSIST_ABORT);
             }
             return !__syncthreads_or(gave_up);
+        }
+
+        // The first barrier of a launch also finds out whether every CTA has an SM. The launch is a plain one:
+        // a cooperative one waits, holding up the launches of every other stream as well, until the whole
+        // device is free, and a kernel of another library may keep one SM for long. So a CTA that has waited
+        // for `ARRIVE_POLLS` (some 0.1 ms) calls the launch off. That and the last arrival are decided by the
+        // same word, so either all go on, each with its SM, or all leave, having changed nothing that
+        // counts (PERSIST_LATE tells the host). 20^3 beside a one-CTA kernel of 200 ms: 199 ms for a
+        // cooperative launch and 189 ms for a small kernel of a third stream; now 2.6 and 0.07 ms.
+        constexpr int ARRIVE_POLLS = 256;
+
+        __device__ __forceinline__ bool ps_begin(unsigned *bar, unsigned &target)
+        {
+            ps_arrive(bar);
+            target += gridDim.x;
+            bool leave = false;
+            if (threadIdx.x == 0)
+            {
+                unsigned v = ld_acquire_gpu(bar);
+#pragma unroll 1
+                for (int i = 0; i < ARRIVE_POLLS && v < target; ++i)
+                    v = ld_acquire_gpu(bar); // the abort bit ends the wait too
+                // (At most one round per arrival: only those change the word while v < target.)
+#pragma unroll 1
+                while (v < target)
+                {
+                    const unsigned seen = atomicCAS(bar, v, v | PERSIST_ABORT | PERSIST_LATE);
+                    if (seen == v)
+                        break;
+                    v = seen;
+                }
+                leave = (ld_acquire_gpu(bar) & PERSIST_ABORT) != 0;
+            }
+            return !__syncthreads_or(leave);
         }
 
         __device__ __forceinline__ bool ps_barrier(unsigned *bar, unsigned &target, long long limit)
@@ -613,7 +648,9 @@ namespace pmas
             }
             // x is where the first residual gathers it once every CTA is past this barrier (which also
             // orders the table above).
-            ok = ps_barrier(a.bar, target, a.cfg.wait_limit) && ok;
+            ok = ps_begin(a.bar, target) && ok;
+            if (tid == 0)
+                sh.began = ok; // (kept here, not in a register through the loop)
 
 #pragma unroll 1
             for (int n = a.first ? -1 : 0; ok; ++n)
@@ -988,10 +1025,11 @@ namespace pmas
                 ok = ps_barrier(a.bar, target, a.cfg.wait_limit);
             }
 
-            // ---- Out: x, r, the state; no copy may be in flight when the CTA leaves.
+            // ---- Out: x, r, the state (as they were where the launch did not begin); no copy may be in flight
+            // when the CTA leaves.
             __syncthreads();
 #pragma unroll 1
-            for (int j = w; j < nb; j += PS_WARPS)
+            for (int j = w; sh.began && j < nb; j += PS_WARPS)
 #pragma unroll 1
                 for (int e = lane; e < N; e += 32)
                 {
@@ -1010,7 +1048,7 @@ namespace pmas
                     for (long long i = 0; i < MBAR_SPIN_LIMIT; ++i)
                         if (mbar_try_wait(&sh.ring_bar[g % buffers], (uint32_t)(g / buffers) & 1u))
                             break;
-                if (blockIdx.x == 0)
+                if (sh.began && blockIdx.x == 0)
                     *a.st = sh.st;
             }
         }
@@ -1132,10 +1170,8 @@ namespace pmas
     bool prepare_persistent(int bd, int storage)
     {
         return dispatch_variant(bd, storage, [&]<int BD, class Store>() {
-            int coop = 0, dev = 0, per_sm = 0;
-            cudaGetDevice(&dev);
-            if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-                cudaFuncSetAttribute(k_pcg_persistent<BD, Store>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            int per_sm = 0;
+            if (cudaFuncSetAttribute(k_pcg_persistent<BD, Store>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)PS_SMEM) != cudaSuccess ||
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_persistent<BD, Store>, PS_THREADS,
                                                               PS_SMEM) != cudaSuccess ||
@@ -1180,10 +1216,8 @@ namespace pmas
         a.period = period;
         cuda_check(cudaMemsetAsync(bar, 0, sizeof(unsigned), s), "barrier reset");
         dispatch_variant(mas.bd, mas.storage, [&]<int BD, class Store>() {
-            void *args[] = {&a};
-            cuda_check(cudaLaunchCooperativeKernel((const void *)k_pcg_persistent<BD, Store>, dim3(pl.grid),
-                                                   dim3(PS_THREADS), args, pl.smem, s),
-                       "persistent solve launch");
+            k_pcg_persistent<BD, Store><<<pl.grid, PS_THREADS, pl.smem, s>>>(a);
+            cuda_check(cudaGetLastError(), "persistent solve launch");
         });
     }
 } // namespace pmas
