@@ -390,6 +390,7 @@ struct mas_solver
     bool graph_aligned = false;
     bool capturing = false;
     std::vector<std::pair<int, long long>> graph_counts[2]; // kernels per kind in one replay
+    int graph_captures = 0; // over the handle's life
     int capture_slot = 0;
 
     // Info of the last solve (MASSolver.cu:145-149).
@@ -1068,6 +1069,7 @@ struct mas_solver
         cudaError_t e = cudaGraphInstantiate(&graph_exec[slot], graph, 0);
         cudaGraphDestroy(graph);
         cuda_check(e, "graph instantiate");
+        ++graph_captures;
     }
 
     void ensure_graph(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, int P, int chunk)
@@ -1090,7 +1092,6 @@ struct mas_solver
         mix((uint64_t)chained_launch());
         mix((uint64_t)spmv_unroll());
         mix((uint64_t)apply_items_per_warp());
-        mix((uint64_t)Av.keep);
         uint64_t bits;
         std::memcpy(&bits, &cfg.rel_tol, 8);
         mix(bits);
@@ -1166,8 +1167,7 @@ struct mas_solver
     // pcg_solve (MASSolver.cu:469-595) on device-resident b_ / x_ (padded order).
     void pcg()
     {
-        BankedView Av = A.view();
-        Av.keep = kept_banks();
+        const BankedView Av = A.view();
         const MasView mv = mas.view();
         const PcgConfig cfg = config();
         cudaEvent_t e0, e1;
@@ -1239,7 +1239,7 @@ struct mas_solver
     void pcg_start(const BankedView &Av, const MasView &mv, const PcgConfig &cfg)
     {
         PcgState *S = st.get();
-        launch_pcg_init_state(S, stream);
+        launch_pcg_init_state(S, kept_banks(), stream);
         // r = b - A x, rr0, the level-0 restriction of r, then z = M^-1 r
         run("spmv_residual", 1, [&] { launch_spmv(SPMV_RESIDUAL, Av, x.get(), r.get(), b.get(), S, red(), 0, 0, stream); });
         run("restrict", 0, [&] { return launch_restrict(mv, r.get(), S, 0, stream); });
@@ -2210,6 +2210,7 @@ struct mas_solver
             o.obj.emplace_back("factorize_phases_ms", fp);
         }
         o.obj.emplace_back("launched_iterations", num(launched_iterations, true));
+        o.obj.emplace_back("graph_captures", num(graph_captures, true));
         o.obj.emplace_back("banks", num(banks, true));
         o.obj.emplace_back("coarse_levels", num(mas.level_num, true));
         o.obj.emplace_back("kernel_launches_total", num((double)total_launches, true));
