@@ -1056,19 +1056,24 @@ namespace pmas
         constexpr size_t PS_SMEM = 232448 - 1024; // dynamic shared memory beside the static part
         static_assert(sizeof(PsShared) <= 1024, "static shared memory of the persistent solve");
 
-        // Banks up to which one launch is the faster way: beyond, an SM's 12 warps are busy with products
-        // for longer than the iteration kernels' launches cost. us per iteration, one launch / iteration
-        // kernels, on both sides of each line: 3 x 3 blocks FP64 38.5 / 39.9 at 1,350 banks and 42.8 / 40.1
-        // at 1,470, FP32 36.1 / 41.5 at 1,716 and 43.3 / 42.4 at 1,855, binary16 29.6 / 36.6 at 1,584 and
-        // 37.4 / 37.3 at 1,855; 2 x 2 FP64 26.0 / 28.6 at 1,670 and 30.5 / 29.8 at 1,930, FP32 27.6 / 27.7 at
-        // 2,220 and 31.5 / 30.1 at 2,519, binary16 28.2 / 28.4 at 2,519; scalar FP64 23.7 / 25.8 at 3,050 and
-        // 28.6 / 26.5 at 3,680, FP32 and binary16 28.2 / 29.2 and 28.1 / 28.7 at 4,930.
+        // Banks up to which one launch is the faster way: beyond, an SM's 12 warps are busy with products for
+        // longer than the iteration kernels' launches cost. With 148 SMs of 12 warps the time rises by steps:
+        // every 1,776 banks one more round of products, every 148 one more bank on an SM. us per iteration, one launch /
+        // iteration kernels, on both sides of each line: 3 x 3 blocks FP32 35.1 / 39.2 at 1,716 banks and
+        // 42.7 / 39.7 at 1,855, binary16 36.5 / 35.9 at 1,855, 37.1 / 37.7 at 2,000 (29.5 / 35.4 at 1,716); 2 x 2
+        // FP64 27.5 / 29.2 at 1,718 and 30.4 / 29.3 at 1,871, FP32 27.6 / 27.7 at 2,220 and 31.3 / 28.0 at 2,275,
+        // binary16 26.9 / 27.4 at 2,275, 27.9 / 27.8 at 2,395 and 28.9 / 28.1 at 2,519; scalar FP64 23.1 / 24.9
+        // at 3,042, 23.6 / 26.5 at 3,456 and 28.6 / 26.5 at 3,680, FP32 29.2 / 29.4 at 4,921 and 32.2 / 29.0 at 5,200,
+        // binary16 28.4 / 28.8 at 5,200 and 30.1 / 28.1 at 5,488. (3 x 3 FP64: 38.5 / 39.9 at 1,350, where
+        // the plan below still finds room for the inverses; for a cube of 1,341 banks it does not.)
         template <int BD, class Store>
         constexpr int persist_max_banks()
         {
             if (std::is_same_v<Store, double>)
-                return BD == 3 ? 1400 : (BD == 2 ? 1800 : 3200);
-            return BD == 3 ? (std::is_same_v<Store, float> ? 1800 : 1900) : (BD == 2 ? 2300 : PERSIST_MAX_BANKS);
+                return BD == 3 ? 1400 : (BD == 2 ? 1776 : 3200);
+            if (std::is_same_v<Store, float>)
+                return BD == 3 ? 1776 : (BD == 2 ? 2220 : 4930);
+            return BD == 3 ? 1900 : (BD == 2 ? 2300 : PERSIST_MAX_BANKS);
         }
 
         template <int BD, class Store>
