@@ -318,49 +318,9 @@ namespace
     std::atomic<bool> OneLaunchTurn::taken[64];
 } // namespace
 
-namespace
-{
-    // The memory pool a handle factorizes with (AllocScope). It holds on to KEEP bytes, the handle's live
-    // buffers among them: freed temporaries of smaller systems stay in it for the next factorization, those
-    // that would bring it above go back to the device at the next wait for the stream, and so does
-    // everything at the handle's end or when an allocation fails anywhere (device_alloc). Declared before
-    // the handle's buffers, so it is destroyed after them.
-    struct AllocPool
-    {
-        static constexpr uint64_t KEEP = 256ull << 20;
-        cudaMemPool_t pool = nullptr;
-        cudaMemPool_t get(int device)
-        {
-            if (pool)
-                return pool;
-            cudaMemPoolProps props = {};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = device;
-            if (cudaMemPoolCreate(&pool, &props) != cudaSuccess)
-            {
-                cudaGetLastError();
-                pool = nullptr; // plain allocations then
-                return pool;
-            }
-            uint64_t keep = KEEP;
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-            register_pool(pool, device);
-            return pool;
-        }
-        ~AllocPool()
-        {
-            if (!pool)
-                return;
-            unregister_pool(pool);
-            cudaMemPoolDestroy(pool);
-        }
-    };
-} // namespace
-
 struct mas_solver
 {
-    AllocPool alloc_pool;
+    AllocPoolRef alloc_pool;
     Params p;
     int device = 0;
     cudaStream_t own_stream = nullptr;
@@ -760,7 +720,14 @@ struct mas_solver
             tp = now;
         };
         cuda_check(cudaSetDevice(device), "set device");
-        const AllocScope scope(alloc_pool.get(device), stream);
+        if (!alloc_pool.p)
+            alloc_pool.p = AllocPool::of(device);
+        struct Settle
+        {
+            AllocPool &pool;
+            ~Settle() { pool.settle(); }
+        } const settle{*alloc_pool.p};
+        const AllocScope scope(alloc_pool.p->pool, stream);
         if (declared)
         {
             if (!factorized)

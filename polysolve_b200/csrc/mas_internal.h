@@ -9,6 +9,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <cuda_runtime_api.h>
@@ -64,9 +65,32 @@ namespace pmas
         AllocScope &operator=(const AllocScope &) = delete;
     };
 
-    // The pools whose unused memory a failing allocation gives back (registered while they live).
-    void register_pool(cudaMemPool_t pool, int device);
-    void unregister_pool(cudaMemPool_t pool);
+    // The memory pool that a device's handles factorize with (AllocScope), one for all of them: the driver
+    // enlarges a pool by 32 MB at least, which a pool per handle made the least a handle took (32.5 MB for
+    // 8^3, 96 for 20^3; now 4.5 and 48). Up to KEEP bytes of freed memory stay in it for the next
+    // factorization, counted when one has ended and when a handle goes (settle); all of it goes back to the
+    // device when an allocation fails anywhere (device_alloc), and the pool itself with the last handle.
+    struct AllocPool
+    {
+        static constexpr uint64_t KEEP = 256ull << 20;
+        cudaMemPool_t pool = nullptr; // none: plain allocations
+        explicit AllocPool(int device);
+        ~AllocPool();
+        AllocPool(const AllocPool &) = delete;
+        AllocPool &operator=(const AllocPool &) = delete;
+        static std::shared_ptr<AllocPool> of(int device);
+        void settle();
+    };
+    // A handle's reference; declared before its buffers, so that they are back in the pool when it goes.
+    struct AllocPoolRef
+    {
+        std::shared_ptr<AllocPool> p;
+        ~AllocPoolRef()
+        {
+            if (p)
+                p->settle();
+        }
+    };
 
     // throws Error(ERR_OOM) with MB figures; *pooled: the memory came from the thread's AllocScope
     void *device_alloc(size_t bytes, const char *ctx, bool *pooled);

@@ -15,7 +15,6 @@
 #include <mutex>
 #include <string>
 #include <unordered_map>
-#include <vector>
 
 #include "mas_common.cuh"
 
@@ -48,37 +47,68 @@ namespace pmas
         t_alloc_stream = saved_stream;
     }
 
-    // Every live pool with its device: an allocation that fails gives back what they hold unused.
+    AllocPool::AllocPool(int device)
+    {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess)
+        {
+            cudaGetLastError();
+            pool = nullptr;
+            return;
+        }
+        uint64_t hold = UINT64_MAX; // settle() gives back, not every wait for a stream
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &hold);
+    }
+
+    AllocPool::~AllocPool()
+    {
+        if (pool)
+            cudaMemPoolDestroy(pool);
+    }
+
+    void AllocPool::settle()
+    {
+        uint64_t used = 0;
+        if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+            cudaMemPoolTrimTo(pool, (size_t)used + KEEP);
+        cudaGetLastError();
+    }
+
     static std::mutex g_pools_mutex;
-    static std::vector<std::pair<cudaMemPool_t, int>> g_pools;
+    static std::unordered_map<int, std::weak_ptr<AllocPool>> g_pools; // by device
 
-    void register_pool(cudaMemPool_t pool, int device)
+    std::shared_ptr<AllocPool> AllocPool::of(int device)
     {
         std::lock_guard<std::mutex> lock(g_pools_mutex);
-        g_pools.push_back({pool, device});
+        std::shared_ptr<AllocPool> p = g_pools[device].lock();
+        if (!p)
+            g_pools[device] = p = std::make_shared<AllocPool>(device);
+        return p;
     }
 
-    void unregister_pool(cudaMemPool_t pool)
-    {
-        std::lock_guard<std::mutex> lock(g_pools_mutex);
-        std::erase_if(g_pools, [&](const auto &e) { return e.first == pool; });
-    }
-
-    static void trim_pools()
+    static void trim_pool()
     {
         int device = 0;
         cudaGetDevice(&device);
         if (t_alloc_pool)
             cudaStreamSynchronize(t_alloc_stream); // this thread's own frees
-        std::lock_guard<std::mutex> lock(g_pools_mutex);
-        for (const auto &e : g_pools)
-            if (e.second == device)
-                cudaMemPoolTrimTo(e.first, 0);
+        std::shared_ptr<AllocPool> p;
+        {
+            std::lock_guard<std::mutex> lock(g_pools_mutex);
+            const auto it = g_pools.find(device);
+            if (it != g_pools.end())
+                p = it->second.lock();
+        }
+        if (p && p->pool)
+            cudaMemPoolTrimTo(p->pool, 0);
         cudaGetLastError();
     }
 
     // Allocation with the reference's out-of-memory message (mas_utils/CudaUtils.cuh:68-79). Where it
-    // fails, the unused memory of all pools of the device goes back first and it is tried once more.
+    // fails, the unused memory of the device's pool goes back first and it is tried once more.
     void *device_alloc(size_t bytes, const char *ctx, bool *pooled)
     {
         void *p = nullptr;
@@ -104,7 +134,7 @@ namespace pmas
             if (e != cudaErrorMemoryAllocation || attempt > 0)
                 break;
             cudaGetLastError();
-            trim_pools();
+            trim_pool();
         }
         if (e != cudaErrorMemoryAllocation)
             cuda_check(e, ctx);

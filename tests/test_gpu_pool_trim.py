@@ -1,8 +1,10 @@
-"""Memory that the handles' pools hold unused is not missing to others: an allocation of the library that
+"""Memory that the handles' pool holds unused is not missing to others: an allocation of the library that
 fails gives it back to the device first. The failure is injected on the host, so it is final here;
 what counts is the memory that is free afterwards."""
 
 from __future__ import annotations
+
+import gc
 
 import numpy as np
 import pytest
@@ -14,41 +16,40 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("failing", ["factorize", "solve_multi"])
-def test_failed_allocation_trims_every_pool(failing):
+def test_failed_allocation_trims_the_pool(failing):
     torch = pytest.importorskip("torch")
-    handles, systems = [], []
-    for k in range(2):
-        system = synthetic.elasticity(22, young_sigma=1.0, jitter=0.2, seed=80 + k)
+
+    def handle(N, factorize=True):
+        system = synthetic.elasticity(N, young_sigma=1.0, jitter=0.2, seed=80 + N)
         s = Solver.create("MAS", "")
         s.set_parameters({"MAS": {"block_dim": 3, "precision": "fp16", "relative_tolerance": 1e-8,
                                   "absolute_tolerance": 0.0}})
         s.set_positions(system.positions)
-        s.factorize(system.scipy())
-        handles.append(s)
-        systems.append(system)
+        if factorize:
+            s.factorize(system.scipy())
+        return s, system
+
+    kept, system = handle(10)
+    # A larger handle comes and goes: the pool, which lives on with the other one, keeps some of its memory.
+    large, _ = handle(30)
+    del large
+    third, other = handle(10, factorize=False)
+    gc.collect()
     torch.cuda.synchronize()
     before = torch.cuda.mem_get_info()[0]
-    # solve_multi allocates outside the pool, factorize inside one.
-    other = synthetic.elasticity(10, young_sigma=1.0, jitter=0.2, seed=82)
-    if failing == "factorize":
-        third = Solver.create("MAS", "")
-        third.set_parameters({"MAS": {"block_dim": 3, "precision": "fp16", "relative_tolerance": 1e-8,
-                                  "absolute_tolerance": 0.0}})
-        third.set_positions(other.positions)
     debug_fail_allocation(0)
     try:
         with pytest.raises(CudaOutOfMemoryError):
-            if failing == "factorize":
+            if failing == "factorize":  # inside the pool
                 third.factorize(other.scipy())
-            else:
-                handles[1].solve_multi(synthetic.rhs(systems[1].n, seed=80, count=4))
+            else:  # outside
+                kept.solve_multi(synthetic.rhs(system.n, seed=80, count=4))
     finally:
         debug_fail_allocation(-1)
-    # The pools hold memory in pieces of 32 MB and give back those without a live buffer: one at least for
-    # each of these handles, whose sorts of 1.5 million entries are gone.
     assert torch.cuda.mem_get_info()[0] > before
-    for s, system in zip(handles, systems):
-        A, b, x = system.scipy(), synthetic.rhs(system.n, seed=81), np.zeros(system.n)
-        s.factorize(system.scipy())
+    A, b, x = system.scipy(), synthetic.rhs(system.n, seed=81), np.zeros(system.n)
+    for s in (kept, third):
+        s.factorize(A)
+        x[:] = 0.0
         s.solve(b, x)
         assert np.linalg.norm(A @ x - b) <= 2e-8 * np.linalg.norm(b)
