@@ -342,15 +342,34 @@ struct mas_solver
     std::vector<std::pair<int, std::pair<float, float>>> timeline; // kind, start ms, end ms (profiled)
 
     // CUDA graphs of `chunk` PCG iterations, replayed until the device flags done. When the
-    // true-residual period is a multiple of the chunk, graph[0] has no true-residual SpMV and
-    // graph[1] recomputes it in its last iteration; otherwise graph[0] launches the (device-gated)
-    // true-residual SpMV in every iteration.
-    cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
-    uint64_t graph_key = 0;
-    bool graph_aligned = false;
-    bool capturing = false;
-    std::vector<std::pair<int, long long>> graph_counts[2]; // kernels per kind in one replay
+    // true-residual period is a multiple of the chunk, exec[0] has no true-residual SpMV and
+    // exec[1] recomputes it in its last iteration; otherwise exec[0] launches the (device-gated)
+    // true-residual SpMV in every iteration. One set for solves that keep part of the matrix in L2 and
+    // one for those that don't (kept_banks: in a batch), so that a handle used both ways keeps both. (The
+    // number of banks in the device state instead, read by every warp of the SpMV, made a solve of 80^3 0.2 to
+    // 0.6 % longer.)
+    struct IterationGraphs
+    {
+        cudaGraphExec_t exec[2] = {nullptr, nullptr};
+        uint64_t key = 0;
+        bool aligned = false;
+        std::vector<std::pair<int, long long>> counts[2]; // kernels per kind in one replay
+        void drop()
+        {
+            for (int i = 0; i < 2; ++i)
+            {
+                if (exec[i])
+                    cudaGraphExecDestroy(exec[i]);
+                exec[i] = nullptr;
+                counts[i].clear();
+            }
+            key = 0;
+        }
+    };
+    IterationGraphs iteration_graphs[2];
     int graph_captures = 0; // over the handle's life
+    bool capturing = false;
+    std::vector<std::pair<int, long long>> graph_counts[2]; // kernels per kind of the capture in progress
     int capture_slot = 0;
 
     // Info of the last solve (MASSolver.cu:145-149).
@@ -459,9 +478,8 @@ struct mas_solver
         }
         for (cudaEvent_t e : ev_pool)
             cudaEventDestroy(e);
-        for (auto &g : graph_exec)
-            if (g)
-                cudaGraphExecDestroy(g);
+        for (IterationGraphs &g : iteration_graphs)
+            g.drop();
         for (auto &g : ggraph)
             if (g)
                 cudaGraphExecDestroy(g);
@@ -996,20 +1014,16 @@ struct mas_solver
     {
         for (int i = 0; i < 2; ++i)
         {
-            if (graph_exec[i])
-                cudaGraphExecDestroy(graph_exec[i]);
-            graph_exec[i] = nullptr;
-            graph_counts[i].clear();
+            iteration_graphs[i].drop();
             if (ggraph[i])
                 cudaGraphExecDestroy(ggraph[i]);
             ggraph[i] = nullptr;
             ggraph_counts[i].clear();
         }
-        graph_key = 0;
         ggraph_key = 0;
     }
 
-    void capture(int slot, const BankedView &Av, const MasView &mv, const PcgConfig &cfg, int P, int chunk,
+    void capture(IterationGraphs &gs, int slot, const BankedView &Av, const MasView &mv, const PcgConfig &cfg, int P, int chunk,
                  bool aligned)
     {
         cudaGraph_t graph = nullptr;
@@ -1032,14 +1046,16 @@ struct mas_solver
             throw;
         }
         capturing = false;
+        gs.counts[slot] = std::move(graph_counts[slot]);
+        graph_counts[slot].clear();
         cuda_check(cudaStreamEndCapture(stream, &graph), "end capture");
-        cudaError_t e = cudaGraphInstantiate(&graph_exec[slot], graph, 0);
+        cudaError_t e = cudaGraphInstantiate(&gs.exec[slot], graph, 0);
         cudaGraphDestroy(graph);
         cuda_check(e, "graph instantiate");
         ++graph_captures;
     }
 
-    void ensure_graph(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, int P, int chunk)
+    IterationGraphs &ensure_graph(const BankedView &Av, const MasView &mv, const PcgConfig &cfg, int P, int chunk)
     {
         uint64_t key = 1469598103934665603ull;
         auto mix = [&key](uint64_t v) {
@@ -1059,6 +1075,7 @@ struct mas_solver
         mix((uint64_t)chained_launch());
         mix((uint64_t)spmv_unroll());
         mix((uint64_t)apply_items_per_warp());
+        mix((uint64_t)Av.keep);
         uint64_t bits;
         std::memcpy(&bits, &cfg.rel_tol, 8);
         mix(bits);
@@ -1066,14 +1083,16 @@ struct mas_solver
         mix(bits);
         mix((uint64_t)P);
         mix((uint64_t)chunk);
-        if (graph_exec[0] && key == graph_key)
-            return;
-        drop_graph();
-        graph_aligned = (P % chunk == 0);
-        capture(0, Av, mv, cfg, P, chunk, graph_aligned);
-        if (graph_aligned)
-            capture(1, Av, mv, cfg, P, chunk, true);
-        graph_key = key;
+        IterationGraphs &gs = iteration_graphs[Av.keep > 0 ? 1 : 0];
+        if (gs.exec[0] && key == gs.key)
+            return gs;
+        gs.drop();
+        gs.aligned = (P % chunk == 0);
+        capture(gs, 0, Av, mv, cfg, P, chunk, gs.aligned);
+        if (gs.aligned)
+            capture(gs, 1, Av, mv, cfg, P, chunk, true);
+        gs.key = key;
+        return gs;
     }
 
     // The shape of the one-launch solve, or one that is not ok: the iteration kernels run instead for
@@ -1134,7 +1153,8 @@ struct mas_solver
     // pcg_solve (MASSolver.cu:469-595) on device-resident b_ / x_ (padded order).
     void pcg()
     {
-        const BankedView Av = A.view();
+        BankedView Av = A.view();
+        Av.keep = kept_banks();
         const MasView mv = mas.view();
         const PcgConfig cfg = config();
         cudaEvent_t e0, e1;
@@ -1206,7 +1226,7 @@ struct mas_solver
     void pcg_start(const BankedView &Av, const MasView &mv, const PcgConfig &cfg)
     {
         PcgState *S = st.get();
-        launch_pcg_init_state(S, kept_banks(), stream);
+        launch_pcg_init_state(S, stream);
         // r = b - A x, rr0, the level-0 restriction of r, then z = M^-1 r
         run("spmv_residual", 1, [&] { launch_spmv(SPMV_RESIDUAL, Av, x.get(), r.get(), b.get(), S, red(), 0, 0, stream); });
         run("restrict", 0, [&] { return launch_restrict(mv, r.get(), S, 0, stream); });
@@ -1225,8 +1245,7 @@ struct mas_solver
         const int P = p.true_residual_period;
         const int chunk = p.poll_period;
         const bool graphs = p.graphs && !p.profile && first == 1;
-        if (graphs)
-            ensure_graph(Av, mv, cfg, P, chunk);
+        const IterationGraphs *gs = graphs ? &ensure_graph(Av, mv, cfg, P, chunk) : nullptr;
         int launched = 0;
         bool stop = false;
         int pending = -1; // slot holding the previous chunk's state copy
@@ -1239,9 +1258,9 @@ struct mas_solver
             const int k1 = std::min(p.max_iter, k0 + chunk - 1);
             if (graphs)
             {
-                const int g = (graph_aligned && (k0 + chunk - 1) % P == 0) ? 1 : 0;
-                cuda_check(cudaGraphLaunch(graph_exec[g], stream), "graph launch");
-                for (auto &gc : graph_counts[g])
+                const int g = (gs->aligned && (k0 + chunk - 1) % P == 0) ? 1 : 0;
+                cuda_check(cudaGraphLaunch(gs->exec[g], stream), "graph launch");
+                for (auto &gc : gs->counts[g])
                 {
                     kstats[gc.first].second.launches += gc.second;
                     total_launches += gc.second;

@@ -146,6 +146,7 @@ namespace pmas
         const int *rowlen;      // nodes
         const int *cols;        // slots * 32, padded node ids
         const double *vals;     // slots * 32 * bd * bd
+        int keep = 0;           // banks below it stay in L2 between products, the others stream through
     };
 
     __host__ __device__ inline long long banked_value_index(long long slot, int lane, int q, int bd)
@@ -323,10 +324,7 @@ namespace pmas
         int x_defer, x_applied;
         // Arrival tickets of the grid reductions: [0] SpMV p.Ap / initial residual, [1] update_xr,
         // [2] in-loop true residual, [4] MAS apply. The last CTA resets its ticket to zero.
-        unsigned int counter[7];
-        // Banks of the matrix that stay in L2 between products (the others stream through); set at the start
-        // of a solve. Here and not a kernel argument, so that the graphs serve solves with any number.
-        int keep;
+        unsigned int counter[8];
     };
 
     // Default iteration limit of a bounded device-side wait (an mbarrier wait of a bulk copy, a grid barrier of
@@ -468,7 +466,7 @@ namespace pmas
                            size_t dst_len, cudaStream_t s);
     void launch_permute_out(int n, int bd, int V, const int *padded_of_block, const double *src, double *dst,
                             cudaStream_t s);
-    void launch_pcg_init_state(PcgState *st, int keep, cudaStream_t s);
+    void launch_pcg_init_state(PcgState *st, cudaStream_t s);
     // Grids of one system's update launches, and the batched launches (every system's state
     // reset to zero by launch_init_states_batch, one CTA per system).
     int update_xr_grid(const MasView &mas);

@@ -390,13 +390,6 @@ namespace pmas
                 dst[i] = __ldcg(src + i);
         }
 
-        __global__ void k_init_state(PcgState *st, int keep)
-        {
-            unsigned *w = reinterpret_cast<unsigned *>(st);
-            for (int i = threadIdx.x; i < (int)(sizeof(PcgState) / sizeof(unsigned)); i += blockDim.x)
-                w[i] = i == (int)(offsetof(PcgState, keep) / sizeof(unsigned)) ? (unsigned)keep : 0u;
-        }
-
         // Every system's PcgState set to zero (the batched form of launch_pcg_init_state).
         __global__ void k_init_states_batch(BatchView v)
         {
@@ -600,9 +593,8 @@ namespace pmas
         cuda_check(cudaGetLastError(), "zero launch");
     }
 
-    void launch_pcg_init_state(PcgState *st, int keep, cudaStream_t s)
+    void launch_pcg_init_state(PcgState *st, cudaStream_t s)
     {
-        k_init_state<<<1, 64, 0, s>>>(st, keep);
-        cuda_check(cudaGetLastError(), "state reset launch");
+        cuda_check(cudaMemsetAsync(st, 0, sizeof(PcgState), s), "state reset");
     }
 } // namespace pmas

@@ -34,12 +34,9 @@ namespace pmas
             const int lane = threadIdx.x & 31;
             const int bank = cta.x * BANKS_PER_CTA + warp_index();
             const int u = bank * 32 + lane;
-            // The matrix is not written during a solve, nor is st->keep after its start: the row ends and (in the
-            // loop) the load policy come before the wait.
+            // The matrix is not written during a solve: its row ends come before the wait.
             long long s0 = 0;
-            int len = 0, keep = 0;
-            if (MODE == SPMV_PAP)
-                keep = __ldcg(&st->keep);
+            int len = 0;
             if (bank < A.banks)
             {
                 s0 = A.slice[bank];
@@ -51,8 +48,6 @@ namespace pmas
                 st->x_applied = st->x_defer;
             if (MODE != SPMV_PLAIN && st->done)
                 return;
-            if (MODE == SPMV_RESIDUAL)
-                keep = st->keep;
             // In-loop true residual: only every `period`-th iteration (iteration = st->iter + 1).
             if (MODE == SPMV_RESIDUAL && period > 0 && (st->iter + 1) % period != 0)
                 return;
@@ -66,9 +61,9 @@ namespace pmas
                 for (int i = 0; i < BD; ++i)
                     acc[i] = 0.0;
                 // The matrix streams through L2 with evict-first priority (x, the gathered vector,
-                // and the other PCG vectors stay resident), but for its first st->keep banks where the
+                // and the other PCG vectors stay resident), but for its first A.keep banks where the
                 // vectors leave room (kept_banks); two slots' loads in flight per lane.
-                const uint64_t pol = bank < keep ? l2_evict_normal_policy() : l2_evict_first_policy();
+                const uint64_t pol = bank < A.keep ? l2_evict_normal_policy() : l2_evict_first_policy();
                 if constexpr (BD == 1 && UNROLL > 1)
                 {
                     // Scalar rows: four times as many slots for the same bytes in flight, and the last

@@ -1,5 +1,5 @@
-"""A handle's captured iterations serve its solves alone and in batches alike: alternating between the two
-captures nothing anew (what stays in L2 differs between them, but is no part of the graphs)."""
+"""A handle's captured iterations are kept for its solves alone and for those in batches (what stays in L2
+differs between the two): alternating captures nothing anew."""
 
 from __future__ import annotations
 
@@ -23,18 +23,19 @@ def test_alternating_solve_and_batch_keeps_the_graphs(block_dim, N):
             s.set_positions(system.positions)
         s.factorize(system.scipy())
         pairs.append((s, synthetic.rhs(system.n, seed=k)))
-    refs, captures = [], []
+    refs = []
     for s, b in pairs:
         refs.append(np.zeros_like(b))
         s.solve(b, refs[-1])
-        captures.append(s.get_info()["graph_captures"])
-        assert captures[-1] >= 1
-    for _ in range(3):
+    captures = None
+    for _ in range(4):
         xs = [np.zeros_like(b) for _, b in pairs]
         solve_batch([s for s, _ in pairs], [b for _, b in pairs], xs)
-        for (s, b), x, ref, count in zip(pairs, xs, refs, captures):
+        for (s, b), x, ref in zip(pairs, xs, refs):
             np.testing.assert_array_equal(x, ref)
             x[:] = 0.0
             s.solve(b, x)
             np.testing.assert_array_equal(x, ref)
-            assert s.get_info()["graph_captures"] == count
+        now = [s.get_info()["graph_captures"] for s, _ in pairs]
+        assert min(now) >= 1 and (captures is None or now == captures)
+        captures = now
