@@ -33,6 +33,17 @@ namespace pmas
         // same over banks of isolated rows, rc.zc and rc.zc_old over the coarse matrices.
         constexpr int APPLY_PARTS = 6;
 
+        // Whether the solve has stopped, for a whole CTA; read past L1 (see mas_apply_body) and once, not by each
+        // of some 2,000 warps from the same line.
+        __device__ __forceinline__ bool solve_done(const PcgState *st)
+        {
+            __shared__ int stop;
+            if (threadIdx.x == 0)
+                stop = __ldcg(&st->done);
+            __syncthreads();
+            return warp_uniform(stop) != 0;
+        }
+
         // Work item m: m < banks -> level-0 matrix m (input r, output z0); otherwise coarse matrix
         // g = coarse_active[m - banks] (matrix banks + g, input rc, output zc, 32 coarse nodes
         // from g * 32). mode 0: plain apply; 1: initial PCG apply (rz0); 2: PCG iteration.
@@ -94,7 +105,7 @@ namespace pmas
             // for the predecessor (launched chained in a PCG iteration), or at the first coarse matrix.
             if (!early)
                 pdl_wait();
-            if (MODE != 0 && __ldcg(&st->done))
+            if (MODE != 0 && solve_done(st))
             {
                 if (lane == 0)
                     mbar_drain(bar, pending, {0u, 0u});
@@ -303,7 +314,7 @@ namespace pmas
             // for the predecessor (launched chained in a PCG iteration), or at the first coarse matrix.
             if (!early)
                 pdl_wait();
-            if (MODE != 0 && __ldcg(&st->done))
+            if (MODE != 0 && solve_done(st))
             {
                 if (loader)
                     mbar_drain(bar, pending, {0u, 0u});

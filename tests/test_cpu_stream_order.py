@@ -41,7 +41,7 @@ def test_early_apply_reads_past_l1(form):
     text = _code((CSRC / "mas_apply.cu").read_text())
     start = text.index(f"bool {form}(")
     body = text[start:text.index("return true;", start)]
-    assert "__ldcg(&st->done)" in body
-    assert re.findall(r"(?<!__ldcg\(&)st->done", body) == []
+    assert "solve_done(st)" in body and "st->done" not in body
+    assert re.findall(r"bool solve_done\(.*?stop = __ldcg\(&st->done\);", text, flags=re.S)
     assert "__ldcg(in + " in body
     assert re.findall(r"\bin\[", body) == []
