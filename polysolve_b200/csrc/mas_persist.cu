@@ -26,6 +26,7 @@
 // 5,000 for the coarse levels.
 
 #include <algorithm>
+#include <climits>
 
 #include "mas_apply.cuh"
 
@@ -65,6 +66,7 @@ namespace pmas
             int first;      // start the solve (otherwise go on from st, x, r, p)
             int iters;      // iterations of this launch at most
             int period;     // true-residual period (0: never)
+            int polls;      // limit of a grid barrier's wait
         };
 
         // Shared-memory record of one work item. Coarse matrices use r (input) and yz (output) only.
@@ -109,7 +111,7 @@ namespace pmas
             asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
         }
 
-        // Grid barrier: arrive, then wait, for at most `limit` polls (some 0.5 us each). Monotonic arrival
+        // Grid barrier: arrive, then wait, for `limit` polls (some 0.5 us each) after the first. Monotonic arrival
         // count (no reset inside a launch); its top bit (PERSIST_ABORT) tells every CTA that one gave up. A
         // wait that runs out sets it too, and it is the only record of that: the others may be past the
         // barrier by then, and through with the solve.
@@ -120,15 +122,15 @@ namespace pmas
                 red_release_gpu(bar, 1u);
         }
 
-        __device__ __forceinline__ bool ps_wait(unsigned *bar, unsigned &target, long long limit)
+        __device__ __forceinline__ bool ps_wait(unsigned *bar, unsigned &target, int limit)
         {
             target += gridDim.x;
             bool gave_up = false;
             if (threadIdx.x == 0)
             {
-                unsigned v = 0;
+                unsigned v = ld_acquire_gpu(bar);
 #pragma unroll 1
-                for (long long i = 0; i < limit && v < target; ++i)
+                for (int left = limit; v < target && left > 0; --left)
                     v = ld_acquire_gpu(bar); // the abort bit ends the wait too
                 gave_up = v < target || (v & PERSIST_ABORT);
                 if (gave_up)
@@ -171,7 +173,7 @@ namespace pmas
             return !__syncthreads_or(leave);
         }
 
-        __device__ __forceinline__ bool ps_barrier(unsigned *bar, unsigned &target, long long limit)
+        __device__ __forceinline__ bool ps_barrier(unsigned *bar, unsigned &target, int limit)
         {
             ps_arrive(bar);
             return ps_wait(bar, target, limit);
@@ -706,7 +708,7 @@ namespace pmas
                     }
                     if (residual)
                         break;
-                    if (!(ok = ps_barrier(a.bar, target, a.cfg.wait_limit)))
+                    if (!(ok = ps_barrier(a.bar, target, a.polls)))
                         break;
                     stage_dots<0>(dot_pap, bank_pad, 0, bank_pad, staged);
                     __syncthreads();
@@ -750,7 +752,7 @@ namespace pmas
                     }
                     if (!residual)
                         break;
-                    if (!(ok = ps_barrier(a.bar, target, a.cfg.wait_limit)))
+                    if (!(ok = ps_barrier(a.bar, target, a.polls)))
                         break;
                 }
                 if (!ok)
@@ -778,7 +780,7 @@ namespace pmas
                 {
                     if (part == 1)
                     {
-                        if (!(ok = ps_wait(a.bar, target, a.cfg.wait_limit)) || nb == ni)
+                        if (!(ok = ps_wait(a.bar, target, a.polls)) || nb == ni)
                             break;
                         // Coarse levels above the first, four nodes per warp: eight lanes per node, four of its
                         // children each, added in the order of the warp sums of k_coarse_levels (children 16
@@ -897,7 +899,7 @@ namespace pmas
                             dot_rz[team_pad + extra] = beyond;
                     }
                 }
-                if (!(ok = ps_barrier(a.bar, target, a.cfg.wait_limit)))
+                if (!(ok = ps_barrier(a.bar, target, a.polls)))
                     break;
                 // ---- Totals and the scalar step, in every CTA. The coarse corrections of the warp's first
                 // rows of p are on their way meanwhile.
@@ -1022,7 +1024,7 @@ namespace pmas
                 }
                 if (!pdo || n + 1 == a.iters)
                     break;
-                ok = ps_barrier(a.bar, target, a.cfg.wait_limit);
+                ok = ps_barrier(a.bar, target, a.polls);
             }
 
             // ---- Out: x, r, the state (as they were where the launch did not begin); no copy may be in flight
@@ -1219,6 +1221,7 @@ namespace pmas
         a.first = first;
         a.iters = iters;
         a.period = period;
+        a.polls = (int)std::min<long long>(cfg.wait_limit, INT_MAX);
         cuda_check(cudaMemsetAsync(bar, 0, sizeof(unsigned), s), "barrier reset");
         dispatch_variant(mas.bd, mas.storage, [&]<int BD, class Store>() {
             k_pcg_persistent<BD, Store><<<pl.grid, PS_THREADS, pl.smem, s>>>(a);
