@@ -183,7 +183,8 @@ int mas_solve_batch(mas_solver *const *handles, int count, const double *const *
                     const int *n, int device_pointers, int threads, int *statuses);
 
 /* New: solve with device pointers (length n, caller's order) on the handle's stream; the call
- * returns when the solve has finished. */
+ * returns when the solve has finished. (This and mas_solve: a small system's solve is one kernel that keeps
+ * its SMs until it has finished, where they are free and no other solve is in progress on the device.) */
 int mas_solve_device(mas_solver *h, const double *d_b, double *d_x, int n);
 
 /* New: run the handle's device work on the caller's CUDA stream (a cudaStream_t; NULL restores
