@@ -345,7 +345,7 @@ struct mas_solver
     // true-residual period is a multiple of the chunk, exec[0] has no true-residual SpMV and
     // exec[1] recomputes it in its last iteration; otherwise exec[0] launches the (device-gated)
     // true-residual SpMV in every iteration. One set for solves that keep part of the matrix in L2 and
-    // one for those that don't (kept_banks: in a batch), so that a handle used both ways keeps both. (The
+    // one for those that don't (kept_banks: beside others), so that a handle used both ways keeps both. (The
     // number of banks in the device state instead, read by every warp of the SpMV, made a solve of 80^3 0.2 to
     // 0.6 % longer.)
     struct IterationGraphs
@@ -981,13 +981,14 @@ struct mas_solver
     // 0 / 20 / 30 / 40 / 50 MB kept, an iteration takes 48.0 / 45.6 / 44.1 / 43.2 / 44.6 us at 44^3 (binary16,
     // the rule: 45 MB), 123.8 / 120.7 / 121.8 / 124.8 / 128.6 us at 61^3 (FP64, 25 MB), 43.1 / 42.4 / 40.5 /
     // 41.9 / 39.9 us on a 500 x 500 plane (FP64, 32 MB), and at 80^3, whose vectors fill the L2, 172.5 /
-    // 174.3 us with 0 / 20. (A share of every 32 banks: 45.5 us at 44^3 for 40 MB.) Not in a batch,
-    // whose systems share the L2.
+    // 174.3 us with 0 / 20. (A share of every 32 banks: 45.5 us at 44^3 for 40 MB.) Not in a batch
+    // or for a solve that began beside another one, which share the L2: ms per solve of 44^3 from 1 / 2 / 4
+    // threads with it 2.92 / 2.65 / 2.46, now 2.89 / 2.44 / 2.28 (binary16), two of 56^3 4.54 -> 4.25.
     int kept_banks() const
     {
         const double room = l2_bytes * (7.0 / 16.0) - 5.0 * x.bytes() - 16.0 * 32.0 * banks;
         const double matrix = (double)A.vals.bytes() + (double)A.cols.bytes();
-        if (in_batch || room <= 0.0 || matrix <= 0.0)
+        if (in_batch || !alone || room <= 0.0 || matrix <= 0.0)
             return 0;
         return (int)(banks * std::min(1.0, room / matrix));
     }

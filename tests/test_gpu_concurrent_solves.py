@@ -61,3 +61,40 @@ def test_small_solve_beside_another(other, N, launches):
     small.solve(b, x)
     np.testing.assert_array_equal(x, ref)
     assert _launches(small) == 1
+
+
+def test_large_solves_beside_each_other_share_the_l2():
+    """A solve that keeps part of its matrix in L2 does so alone only: of two that run at the same time one
+    uses its other set of captured iterations, which is then kept beside the first."""
+    pairs = [_factorized(44, 93 + k, relative_tolerance=0.0, max_iter=400, precision="fp16") for k in range(2)]
+    refs = []
+    for s, b in pairs:
+        refs.append(np.zeros_like(b))
+        s.solve(b, refs[-1])
+    alone = [s.get_info()["graph_captures"] for s, _ in pairs]
+
+    def captures_after_solving_together():
+        for _ in range(4):
+            start = threading.Barrier(2)
+            xs = [np.zeros_like(b) for _, b in pairs]
+
+            def work(k):
+                start.wait()
+                pairs[k][0].solve(pairs[k][1], xs[k])
+
+            threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+            for x, ref in zip(xs, refs):
+                np.testing.assert_array_equal(x, ref)
+        return [s.get_info()["graph_captures"] for s, _ in pairs]
+
+    together = captures_after_solving_together()
+    assert sum(together) > sum(alone)
+    for (s, b), ref in zip(pairs, refs):
+        x = np.zeros_like(b)
+        s.solve(b, x)
+        np.testing.assert_array_equal(x, ref)
+    assert all(n <= 2 * a for n, a in zip(captures_after_solving_together(), alone))
