@@ -80,7 +80,9 @@ void mas_destroy(mas_solver *h);
  * mas_solve_batch runs the handle, see there), batch_groups (0..64, default 0 = 1: fused groups of
  * a batch), apply_items_per_warp (1..64, default 1: the fewest inverses per warp of the MAS apply,
  * which sets its grid; more suit batches of small systems, and the dot products' summation
- * grouping follows the grid, so results can differ in the last bits between settings). */
+ * grouping follows the grid, so results can differ in the last bits between settings), one_launch
+ * (bool, default true: a lone solve of a small system is one kernel that keeps its SMs until it has
+ * finished; off for programs whose other streams should go on beside solves; the same bits). */
 int mas_set_parameters(mas_solver *h, const char *params_json);
 
 /* MASSolver::get_info (MASSolver.cu:214-219): writes a JSON object with solver_iter,
@@ -183,8 +185,7 @@ int mas_solve_batch(mas_solver *const *handles, int count, const double *const *
                     const int *n, int device_pointers, int threads, int *statuses);
 
 /* New: solve with device pointers (length n, caller's order) on the handle's stream; the call
- * returns when the solve has finished. (This and mas_solve: a small system's solve is one kernel that keeps
- * its SMs until it has finished, where they are free and no other solve is in progress on the device.) */
+ * returns when the solve has finished. (This and mas_solve: see one_launch above.) */
 int mas_solve_device(mas_solver *h, const double *d_b, double *d_x, int n);
 
 /* New: run the handle's device work on the caller's CUDA stream (a cudaStream_t; NULL restores

@@ -65,6 +65,7 @@ namespace
         // Launch the PCG iteration kernels with programmatic dependent launch (each may become
         // resident while its predecessor drains); false: plain stream order.
         bool chained = true;
+        bool one_launch = true;
         // Iterations of each bounded device-side wait before the solve stops with MAS_ERR_TIMEOUT
         // (0: every wait gives up at once -- the test of the timeout path).
         long long wait_limit = MBAR_SPIN_LIMIT_DEFAULT;
@@ -136,7 +137,7 @@ namespace
                                 "true_residual_period", "check_period", "initial_guess", "beta", "ordering",
                                 "poll_period", "profile_kernels", "cuda_graphs", "preconditioner_refresh",
                                 "device_wait_limit", "rhs_group", "chained_launch", "wide_apply", "spmv_unroll",
-                                "batch_launch", "batch_groups", "apply_items_per_warp"};
+                                "batch_launch", "batch_groups", "apply_items_per_warp", "one_launch"};
 
     // MASSolverImpl::set_parameters (MASSolver.cu:198-212) plus the extension keys.
     void apply_mas_params(Params &p, const Json &m, bool strict)
@@ -216,6 +217,8 @@ namespace
             q.graphs = get_bool(*v, "cuda_graphs");
         if (auto *v = m.find("chained_launch"))
             q.chained = get_bool(*v, "chained_launch");
+        if (auto *v = m.find("one_launch"))
+            q.one_launch = get_bool(*v, "one_launch");
         if (auto *v = m.find("spmv_unroll"))
         {
             q.spmv_unroll = get_int(*v, "spmv_unroll");
@@ -1098,12 +1101,12 @@ struct mas_solver
 
     // The shape of the one-launch solve, or one that is not ok: the iteration kernels run instead for
     // larger systems, Polak-Ribiere (its r.z_old dots), per-kernel profiling, host-launched iterations
-    // (cuda_graphs off), and in batches and (but for the smallest) beside other solves, whose kernels fill
+    // (cuda_graphs off), where the caller says so (one_launch off), and in batches and (but for the smallest) beside other solves, whose kernels fill
     // the device.
     PersistPlan persistent_plan(const MasView &mv, const PcgConfig &cfg) const
     {
         PersistPlan pl;
-        if (persist_ready && p.graphs && !p.profile && !in_batch && !cfg.polak_ribiere && p.max_iter >= 1)
+        if (persist_ready && p.one_launch && p.graphs && !p.profile && !in_batch && !cfg.polak_ribiere && p.max_iter >= 1)
             pl = persist_plan(mv);
         if (pl.ok && !alone && pl.grid > device_sm_count() / 4)
             pl.ok = false;

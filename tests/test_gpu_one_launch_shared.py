@@ -96,3 +96,20 @@ def test_long_solve_loses_its_sms_between_launches(block_dim, N):
         print(info["kernel_launches"])
     np.testing.assert_array_equal(got[0][0], got[1][0])
     assert got[0][1:] == got[1][1:]
+
+
+def test_one_launch_off():
+    """The parameter that keeps a program's other streams going beside its solves: captured iterations, the same
+    bits."""
+    s, b = _factorized(14, 98)
+    got = []
+    for on in (True, False, True):
+        s.set_parameters({"MAS": {"one_launch": on}})
+        x = np.zeros_like(b)
+        s.solve(b, x)
+        info = s.get_info()
+        assert info["kernel_launches"].get("pcg_persistent", 0) == int(on)
+        got.append((x, info["solver_iter"], info["solver_error"]))
+    for g in got[1:]:
+        np.testing.assert_array_equal(g[0], got[0][0])
+        assert g[1:] == got[0][1:]
